@@ -23,7 +23,6 @@ struct Gas {
   R gm1;      // gama - 1.0
   R gamaRg;   // gama * Rg   (the reference's left-to-right "gama*Rg*T")
   R inv_Rg;   // 1 / Rg      (fast builds)
-  R inv_gm1;  // 1 / (gama - 1)
   R gam_gm1;  // gama / (gama - 1)  (fast builds: h = gam_gm1 p/rho + |u|^2/2)
   R two_gama; // 2 gama              (fast builds: the all-speed Mach number)
 };
@@ -167,16 +166,11 @@ template <int LIM, typename R>
 __device__ __forceinline__ R limited_slope(R a, R b) {
   const R ab = a * b;
   if (LIM == LIM_MINMOD) return (ab > R(0)) ? R(0.5) * (fabs(b) < fabs(a) ? b : a) : R(0);
-  if (sizeof(R) == 4) {
-    // FP32: one MUFU reciprocal, cheaper than a branch; the select discards
-    // the cases where a + b may vanish
-    const R s = ab * FastMath<R>::rcp(a + b);
-    return (ab > R(0)) ? s : R(0);
-  }
-  // FP64: the Newton-refined reciprocal is long, and uniform regions
-  // (a = b = 0) skip it warp-wide
-  if (!(ab > R(0))) return R(0);
-  return ab * FastMath<R>::rcp1(a + b);
+  // no branch: the chains of a cell's four components interleave, and the
+  // select discards the cases where a + b may vanish (a branch that skipped
+  // the FP64 reciprocal in uniform regions serialised the four)
+  const R s = ab * FastMath<R>::rcp1(a + b);
+  return (ab > R(0)) ? s : R(0);
 }
 
 // The reference's explicit one-sided reconstructions, used for faces whose

@@ -307,6 +307,8 @@ void fill_case_const(const ibgpu_case *cs, CaseConst &k) {
   k.gm1 = cs->gama - 1.0;
   k.gamaRg = cs->gama * cs->Rg;
   k.inv_Rg = 1.0 / cs->Rg;
+  k.gam_gm1 = k.gama / k.gm1;
+  k.two_gama = 2.0 * k.gama;
   k.Cp = cs->Cp;
   k.p_ref = cs->p_ref;
   k.area_ref = cs->area_ref;
@@ -1187,8 +1189,8 @@ void stage_args(const ibgpu_ctx *ctx, int k, StageArgs &sa) {
     sa.v.sout[f] = fin ? nullptr : ctx->d_buf[k & 1][f];
   }
   sa.v.tp = cs.tp[k];
-  // one wave of resident stage CTAs (4 per SM FP64, 6 mixed)
-  sa.prefetch = ctx->nsm * (cs.precision == IBGPU_MIXED ? 6 : 4);
+  // one wave of resident stage CTAs (4 per SM FP64, 5 mixed)
+  sa.prefetch = ctx->nsm * (cs.precision == IBGPU_MIXED ? 5 : 4);
 }
 
 int64_t marched_cells(const ibgpu_ctx *ctx, int ts) {

@@ -63,10 +63,12 @@ struct StageThreads {
 };
 
 // Resident CTAs per SM the register budget is fixed for, by arithmetic and
-// block shape (the batched stage tunes between 256 and 288 threads).
+// block shape (the batched stage tunes between 256 and 288 threads).  FP64
+// 56 registers; FP32 48, as 40 (six CTAs) spilled: 20 steps of the 2048^2
+// vortex 8.80 ms with six, 8.35 with five, 9.14 with four.
 template <typename R, int NT>
 constexpr int stage_min_blocks() {
-  return sizeof(R) == 8 ? 4 : (NT > kTileCells ? 5 : 6);
+  return sizeof(R) == 8 ? 4 : (NT > kTileCells ? 4 : 5);
 }
 
 // Residual max-norm of a block of up to 9 warps into the step's diag: warp and
@@ -99,51 +101,54 @@ __device__ __forceinline__ void block_resnorm(const unsigned long long (&rb)[4],
 
 // CFL bound of one normal cell, NS_Solver::Comptdt (NS_Solver.cpp:196-280),
 // with every operation separately rounded so the CFL pass and the final
-// stages that fold it in produce the same bits in every build.
-__device__ __forceinline__ double cfl_cell_bound(double T, double u, double v, const LevelConst &L,
-                                                 const CaseConst &cc) {
+// stages that fold it in produce the same bits in every build: cfl_vol over
+// the sum of the cell's wave speeds times face areas.
+__device__ __forceinline__ double cfl_cell_sum(double T, double u, double v, const LevelConst &L,
+                                               const CaseConst &cc) {
   const double c = __dsqrt_rn(__dmul_rn(cc.gamaRg, T));
   const double c0 = __dmul_rn(__dadd_rn(fabs(u), c), L.area_x);
   const double c1 = __dmul_rn(__dadd_rn(fabs(v), c), L.area_y);
   const double c2 = __dmul_rn(__dadd_rn(0.0, c), L.area_z);
-  return __ddiv_rn(L.cfl_vol, __dadd_rn(__dadd_rn(c0, c1), c2));
+  return __dadd_rn(__dadd_rn(c0, c1), c2);
+}
+__device__ __forceinline__ double cfl_cell_bound(double T, double u, double v, const LevelConst &L,
+                                                 const CaseConst &cc) {
+  return __ddiv_rn(L.cfl_vol, cfl_cell_sum(T, u, v, L, cc));
 }
 
-// Block minimum of one positive double per thread (as bits) into *dst, one
-// atomic per block (result unused: not waited for); every thread of the
-// block calls it; sred is shared scratch of NT/32 words nobody else uses
-// meanwhile.
-template <int NT>
-__device__ __forceinline__ void block_min_bits(unsigned long long b, unsigned long long *dst,
-                                               unsigned long long *sred) {
-  b = warp_min_u64(b);
-  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < NT / 32; ++k) b = sred[k] < b ? sred[k] : b;
-    atomicMin(dst, b);  // result unused: a reduction the CTA does not wait for
-  }
-}
-
-// The next step's CFL pass folded into a final stage: the bound of each
-// normal cell from the state this stage wrote (cb >= 0) or, for a normal
-// cell it did not write, from the step state; block minimum into
-// diag->cfl_next_bits.  All threads call it (own = the thread owns a cell).
+// The next step's CFL pass folded into a final stage: the sum of each
+// normal cell from the state this stage wrote (cs >= 0) or, for a normal
+// cell it did not write, from the step state; the tile's smallest bound into
+// diag->cfl_next_bits.  A tile has one level and a rounded quotient falls as
+// its divisor grows, so the smallest bound is cfl_vol over the largest sum,
+// bit for bit: one division per CTA instead of one per cell.  All threads
+// call it (own = the thread owns a cell).
 template <int NT>
 __device__ __forceinline__ void fold_next_cfl(const StageArgs &a, const LevelConst &L,
                                               const CaseConst &cc, uint8_t fl, int64_t slot,
-                                              double cb, unsigned long long *sred, int phase,
+                                              double cs, unsigned long long *sred, int phase,
                                               bool own = true) {
-  double best = 10000.0;
+  unsigned long long m = 0ull;
   if (own && (fl & CF_NORMAL)) {
-    const double d0 =
-        cb >= 0.0 ? cb : cfl_cell_bound(a.s0[F_T][slot], a.s0[F_U][slot], a.s0[F_V][slot], L, cc);
-    if (d0 < 0.0) raise_error(a.diag, phase, ERR_CFL_NEG_DT, (int)slot);
-    best = (d0 < best) ? d0 : best;
+    const double s =
+        cs >= 0.0 ? cs : cfl_cell_sum(a.s0[F_T][slot], a.s0[F_U][slot], a.s0[F_V][slot], L, cc);
+    // a NaN sum bounds nothing (std::min(CFL_dt, CFL_dt0) ignores it)
+    if (s > 0.0) {
+      m = (unsigned long long)__double_as_longlong(s);
+      if (L.cfl_vol < 0.0) raise_error(a.diag, phase, ERR_CFL_NEG_DT, (int)slot);
+    }
   }
   __syncthreads();  // sred is free again (block_resnorm read it)
-  block_min_bits<NT>((unsigned long long)__double_as_longlong(best), &a.diag->cfl_next_bits,
-                     sred + 64);
+  sred += 64;
+  m = warp_max_u64(m);
+  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < NT / 32; ++k) m = sred[k] > m ? sred[k] : m;
+    const double d0 = __ddiv_rn(L.cfl_vol, __longlong_as_double((long long)m));
+    if (m != 0ull && d0 >= 0.0 && d0 < 10000.0)
+      atomicMin(&a.diag->cfl_next_bits, (unsigned long long)__double_as_longlong(d0));
+  }
 }
 
 // One stage of the multistage update for one tile per CTA (256 threads):
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(kTileCells) stage_kernel(StageArgs a, CaseCons
   const int64_t slot = (int64_t)tile * kTileCells + tid;
   const uint8_t fl = sfl[(ly + kHalo) * kReg + (lx + kHalo)];
   unsigned long long rb[4] = {0ull, 0ull, 0ull, 0ull};
-  double cb = -1.0;  // next step's CFL bound of this cell, when this stage writes it
+  double cb = -1.0;  // the cell's sum for the next step's CFL bound, when this stage writes it
   if ((fl & CF_NORMAL) && (fl & (CF_UPDATE | CF_RESET))) {
     const int xlo = ly * (kTile + 1) + lx, xhi = xlo + 1;
     const int ylo = ly * kTile + lx, yhi = ylo + kTile;
@@ -332,7 +337,7 @@ __global__ void __launch_bounds__(kTileCells) stage_kernel(StageArgs a, CaseCons
 #pragma unroll
       for (int c = 0; c < 4; ++c) rb[c] = (unsigned long long)__double_as_longlong(fabs(res[c]));
     }
-    if (FINAL && a.v.cfl_next && wrote) cb = cfl_cell_bound(nT, nu, nv, L, cc);
+    if (FINAL && a.v.cfl_next && wrote) cb = cfl_cell_sum(nT, nu, nv, L, cc);
   }
   if (FINAL) {
     __shared__ unsigned long long sred[64 + kTileCells / 32];
@@ -341,12 +346,6 @@ __global__ void __launch_bounds__(kTileCells) stage_kernel(StageArgs a, CaseCons
   }
 }
 
-// Fast build of the stage (FP64 with FastMath divisions/roots, or FP32 flux
-// arithmetic for the mixed mode): per-cell limited slopes computed once and
-// shared by the cell's two faces in each direction, divisions replaced by
-// reciprocals.  Faces whose outer stencil cell is missing use the
-// reference's one-sided reconstruction (NS_Solver.H:743-750).  The residual,
-// update and primitive recovery run in FP64 in every mode.
 // Four values of one cell (rho, u, v, p), one limited slope set, or one
 // face flux (mass, x-momentum, y-momentum, energy).  In shared memory an FP32
 // record is one float4; an FP64 record is split over two double2 planes
@@ -372,9 +371,6 @@ struct SRec<float> {
   static __device__ __forceinline__ void st(V *a, int i, int, float x, float y, float z, float w) {
     a[i] = make_float4(x, y, z, w);
   }
-  static __device__ __forceinline__ float *comp(V *a, int i, int, int c) {
-    return reinterpret_cast<float *>(a + i) + c;
-  }
 };
 
 template <>
@@ -390,270 +386,188 @@ struct SRec<double> {
     a[i] = make_double2(x, y);
     a[i + n] = make_double2(z, w);
   }
-  static __device__ __forceinline__ double *comp(V *a, int i, int n, int c) {
-    return reinterpret_cast<double *>(a + i + (c >> 1) * n) + (c & 1);
-  }
 };
 
-// One face of the stencil region: cells rL1 | rR1 (rL2, rR2 one further
-// out), slope records sL, sR; dir 0 = x (normal u), 1 = y (normal v).
-// Reconstructed left/right states of one face; false (states set to a
-// benign 1) when the face carries no flux.
-template <typename R, int LIM, int NQ, int NS>
-__device__ __forceinline__ bool face_recon(const typename SRec<R>::V *sq, const uint8_t *sfl,
-                                           const typename SRec<R>::V *sl, int rL1, int rR1,
-                                           int step, int sL, int sR, bool uni, R (&ls)[4],
-                                           R (&rs)[4]) {
-  using S = SRec<R>;
-  bool active = true, hasL2 = true, hasR2 = true;
-  if (!uni) {
-    const uint8_t fL = sfl[rL1], fR = sfl[rR1];
-    active = (fL & CF_PRESENT) && (fR & CF_PRESENT) && ((fL | fR) & CF_NORMAL);
-    hasL2 = (sfl[rL1 - step] & CF_PRESENT) != 0;
-    hasR2 = (sfl[rR1 + step] & CF_PRESENT) != 0;
-  }
-  if (!active) {
-#pragma unroll
-    for (int c = 0; c < 4; ++c) ls[c] = rs[c] = R(1);
-    return false;
-  }
-  const Q4<R> cL = S::ld(sq, rL1, NQ), cR = S::ld(sq, rR1, NQ);
-  if (hasL2) {
-    const Q4<R> s = S::ld(sl, sL, NS);
-    ls[0] = cL.x + s.x; ls[1] = cL.y + s.y; ls[2] = cL.z + s.z; ls[3] = cL.w + s.w;
-  } else {
-    const Q4<R> o = S::ld(sq, rR1 + step, NQ);
-    ls[0] = muscl_left_fast<LIM>(o.x, cL.x, cR.x);
-    ls[1] = muscl_left_fast<LIM>(o.y, cL.y, cR.y);
-    ls[2] = muscl_left_fast<LIM>(o.z, cL.z, cR.z);
-    ls[3] = muscl_left_fast<LIM>(o.w, cL.w, cR.w);
-  }
-  if (hasR2) {
-    const Q4<R> s = S::ld(sl, sR, NS);
-    rs[0] = cR.x - s.x; rs[1] = cR.y - s.y; rs[2] = cR.z - s.z; rs[3] = cR.w - s.w;
-  } else {
-    const Q4<R> o = S::ld(sq, rL1 - step, NQ);
-    rs[0] = muscl_right_fast<LIM>(cL.x, cR.x, o.x);
-    rs[1] = muscl_right_fast<LIM>(cL.y, cR.y, o.y);
-    rs[2] = muscl_right_fast<LIM>(cL.z, cR.z, o.z);
-    rs[3] = muscl_right_fast<LIM>(cL.w, cR.w, o.w);
-  }
-  return true;
+template <typename R>
+__device__ __forceinline__ Q4<R> add4(const Q4<R> &a, const Q4<R> &b) {
+  return Q4<R>{a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w};
+}
+template <typename R>
+__device__ __forceinline__ Q4<R> sub4(const Q4<R> &a, const Q4<R> &b) {
+  return Q4<R>{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
 }
 
-template <typename R, int LIM, int NQ, int NS>
-__device__ __forceinline__ Q4<R> fast_face(const typename SRec<R>::V *sq, const uint8_t *sfl,
-                                           const typename SRec<R>::V *sl, int rL1, int rR1, int step,
-                                           int sL, int sR, bool xdir, bool uni, const Gas<R> &g,
-                                           R area, R halfarea) {
-  R ls[4], rs[4];
-  Q4<R> out = {R(0), R(0), R(0), R(0)};
-  if (!face_recon<R, LIM, NQ, NS>(sq, sfl, sl, rL1, rR1, step, sL, sR, uni, ls, rs)) return out;
-  // normal / tangential velocity by selection (one flux evaluation even
-  // when the lanes of a warp mix x- and y-faces)
-  R fm, fn, ft, fe;
-  const R lun = xdir ? ls[1] : ls[2], lut = xdir ? ls[2] : ls[1];
-  const R run = xdir ? rs[1] : rs[2], rut = xdir ? rs[2] : rs[1];
-  roe_flux_states<R>(g, area, halfarea, ls[0], lun, lut, ls[3], rs[0], run, rut, rs[3], fm, fn,
-                     ft, fe);
-  out = Q4<R>{fm, xdir ? fn : ft, xdir ? ft : fn, fe};
-  return out;
-}
-
-// Limited slopes of one cell in one direction (zero where a neighbour is
-// missing; such faces take the one-sided reconstruction instead).
-template <typename R, int LIM, int NQ, int NS>
-__device__ __forceinline__ void fast_slope(const typename SRec<R>::V *sq, const uint8_t *sfl,
-                                           typename SRec<R>::V *sl, int di, int rc, int step,
-                                           bool uni) {
+// The states region cell rc (value c) gives to its two faces along `step`:
+// lo to the face towards rc - step, hi to the one towards rc + step.  A cell
+// whose neighbour on one side is missing has a flux only on the other, with
+// the reference's one-sided reconstruction (its stencil then takes the cell
+// two steps away on that side, NS_Solver.H:743-750); states of faces that
+// carry no flux are left unset (c).
+template <typename R, int LIM, int NQ>
+__device__ __forceinline__ void cell_states(const typename SRec<R>::V *sq, const uint8_t *sfl,
+                                            const Q4<R> &c, int rc, int step, bool uni, Q4<R> &lo,
+                                            Q4<R> &hi) {
   using S = SRec<R>;
-  R s0 = R(0), s1 = R(0), s2 = R(0), s3 = R(0);
   if (uni || ((sfl[rc - step] & CF_PRESENT) && (sfl[rc + step] & CF_PRESENT))) {
-    const Q4<R> m = S::ld(sq, rc - step, NQ), c = S::ld(sq, rc, NQ), p = S::ld(sq, rc + step, NQ);
-    s0 = limited_slope<LIM>(c.x - m.x, p.x - c.x);
-    s1 = limited_slope<LIM>(c.y - m.y, p.y - c.y);
-    s2 = limited_slope<LIM>(c.z - m.z, p.z - c.z);
-    s3 = limited_slope<LIM>(c.w - m.w, p.w - c.w);
+    const Q4<R> m = S::ld(sq, rc - step, NQ), p = S::ld(sq, rc + step, NQ);
+    const Q4<R> s = {limited_slope<LIM>(c.x - m.x, p.x - c.x),
+                     limited_slope<LIM>(c.y - m.y, p.y - c.y),
+                     limited_slope<LIM>(c.z - m.z, p.z - c.z),
+                     limited_slope<LIM>(c.w - m.w, p.w - c.w)};
+    lo = sub4(c, s);
+    hi = add4(c, s);
+    return;
   }
-  S::st(sl, di, NS, s0, s1, s2, s3);
+  lo = hi = c;
+  if (sfl[rc - step] & CF_PRESENT) {
+    const Q4<R> m = S::ld(sq, rc - step, NQ), o = S::ld(sq, rc - 2 * step, NQ);
+    lo = Q4<R>{muscl_right_fast<LIM>(m.x, c.x, o.x), muscl_right_fast<LIM>(m.y, c.y, o.y),
+               muscl_right_fast<LIM>(m.z, c.z, o.z), muscl_right_fast<LIM>(m.w, c.w, o.w)};
+  } else if (sfl[rc + step] & CF_PRESENT) {
+    const Q4<R> p = S::ld(sq, rc + step, NQ), o = S::ld(sq, rc + 2 * step, NQ);
+    hi = Q4<R>{muscl_left_fast<LIM>(o.x, c.x, p.x), muscl_left_fast<LIM>(o.y, c.y, p.y),
+               muscl_left_fast<LIM>(o.z, c.z, p.z), muscl_left_fast<LIM>(o.w, c.w, p.w)};
+  }
+}
+
+// Whether the face between cells with flags fL | fR carries a flux.
+__device__ __forceinline__ bool face_active(uint8_t fL, uint8_t fR) {
+  return (fL & CF_PRESENT) && (fR & CF_PRESENT) && ((fL | fR) & CF_NORMAL);
+}
+
+// Flux (mass, x-momentum, y-momentum, energy) of one face from its states:
+// normal / tangential velocity by selection (one flux evaluation even when
+// the lanes of a warp mix x- and y-faces).
+template <typename R>
+__device__ __forceinline__ Q4<R> state_flux(const Gas<R> &g, bool xdir, R area, R halfarea,
+                                            const Q4<R> &l, const Q4<R> &r) {
+  R fm, fn, ft, fe;
+  roe_flux_states<R>(g, area, halfarea, l.x, xdir ? l.y : l.z, xdir ? l.z : l.y, l.w, r.x,
+                     xdir ? r.y : r.z, xdir ? r.z : r.y, r.w, fm, fn, ft, fe);
+  return Q4<R>{fm, xdir ? fn : ft, xdir ? ft : fn, fe};
 }
 
 // Fast build of the stage (FP64 with FastMath divisions/roots, or FP32 flux
-// arithmetic for the mixed mode): per-cell limited slopes computed once and
-// shared by the cell's two faces in each direction, divisions replaced by
-// reciprocals, cell and face records in shared memory as 128-bit vectors,
-// fixed thread-to-cell/face mapping (thread (tx, ty) owns the slopes and the
-// west/south faces of cell (tx, ty); one warp adds the east/north edge).
-// Faces whose outer stencil cell is missing use the reference's one-sided
-// reconstruction (NS_Solver.H:743-750).  The residual, update and primitive
-// recovery run in FP64 in every mode.
-// NT: threads of the CTA, 256 (edge faces on the first two warps) or 288
-// (a ninth warp owns them); the same arithmetic either way.
-template <typename R, int LIM, bool VISC, bool FINAL, typename TI,
-          int NT = StageThreads<R>::value>
-__device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageVar &v,
-                                                const CaseConst &cc,
-                                                const int tile, const int phase,
-                                                const int fold, const int prefetch) {
-  constexpr int kSX = kTile + 2;  // x-slope row length (cols -1..16)
+// arithmetic for the mixed mode).  Thread (tx, ty) owns cell (tx, ty): it
+// limits the cell's slopes in both directions, keeps the states the cell
+// gives to its west and south faces in registers and leaves those it gives
+// to its east and north faces in shared memory; then it evaluates its west
+// and south faces (the face's flux replaces the state it was made from, so
+// one array serves both) and finally gathers the two fluxes its neighbours
+// computed.  One warp adds the edge: the outer cells' states and the east
+// and north faces.  The residual, update and primitive recovery run in FP64
+// in every mode.
+//
+// What bounds it (2048^2 vortex, FP64): the latency of the CTA's chain of
+// load, slopes, faces and update under four resident CTAs, with the FP64 pipe
+// 55 % busy (floor 79 us a stage at 351 FP64 instructions per cell).  Cells
+// held in registers instead of re-read records, states handed over instead
+// of slopes, a halo addressed by whole warps (no divisions by the region
+// width), limiting without branches and one test per tile for uniform tiles
+// took a cell-stage from 896 to 765 instructions: 20 four-stage steps 14.58
+// -> 12.27 ms FP64, 9.15 -> 8.35 ms mixed.  Measured slower: two cells per
+// thread (13.8 ms, mixed 10.6: fewer warps to hide latency), persistent CTAs
+// copying the next region ahead (13.3), U^n copied ahead into shared memory
+// (12.5).
+// NT: threads of the CTA, 256 (the edge on the first warp) or 288 (a ninth
+// warp owns it); the same arithmetic either way.
+// UNI: a uniform tile (it and its four side neighbours hold only leaf cells
+// that recover their primitives): no presence flags, no one-sided stencils,
+// every cell updated; decided once per tile so neither path tests again.
+// nb: the tile this thread's halo lane reads (-1: none).
+template <typename R, int LIM, bool VISC, bool FINAL, typename TI, int NT, bool UNI>
+__device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v,
+                                           const CaseConst &cc, const LevelConst &L,
+                                           const int tile, const int nb, const int phase,
+                                           const int fold, typename SRec<R>::V *sq, uint8_t *sfl,
+                                           typename SRec<R>::V *fx, typename SRec<R>::V *fy) {
   using S = SRec<R>;
   using V = typename S::V;
-  constexpr int NQ = kReg * kReg, NS = kTile * kSX, NF = kTile * (kTile + 1);
-  __shared__ V sq[S::kPlanes * NQ];
-  __shared__ uint8_t sfl[NQ];
-  __shared__ V slx[S::kPlanes * NS];  // rows 0..15, cols -1..16
-  __shared__ V sly[S::kPlanes * NS];  // rows -1..16, cols 0..15
-  __shared__ V fx[S::kPlanes * NF];   // x-face (i, j) at j*17 + i
-  __shared__ V fy[S::kPlanes * NF];   // y-face (i, j) at j*16 + i
-
-  static_assert(NT == kTileCells || NT == kTileCells + 32, "256 or 288 threads");
+  constexpr int kFX = kTile + 1;  // faces of a row
+  constexpr int NQ = kReg * kReg, NF = kTile * kFX;
   const int tid = threadIdx.x;
   const int tx = tid & (kTile - 1), ty = (NT > kTileCells) ? ((tid >> 4) & (kTile - 1)) : (tid >> 4);
   // a cell of the tile (the ninth warp owns none)
   const bool own = (NT > kTileCells) ? tid < kTileCells : true;
-  const int lvl = a.tile_level[tile];
-  const LevelConst &L = cc.lev[lvl];
-  // uniform tile: it and its four side neighbours hold only leaf cells that
-  // recover their primitives, so no presence flags or one-sided stencils
-  const bool uni = a.tile_uniform != nullptr && a.tile_uniform[tile] != 0;
+  // lane of the edge warp, negative on the others
+  const int et = NT > kTileCells ? tid - kTileCells : (tid < 32 ? tid : -1);
 
-  // side neighbours (the centre entry of the table is the tile itself),
-  // loaded beside the tile's level and uniform flag so the region's loads
-  // below wait for one round trip, not one per neighbour lookup
-  const int32_t *nbrow = a.tile_nb + (int64_t)tile * 9;
-  const int nbs = __ldg(nbrow + 1), nbw = __ldg(nbrow + 3), nbe = __ldg(nbrow + 5),
-            nbn = __ldg(nbrow + 7);
-
+  // ---- the region: each thread its own cell, and four whole warps one side
+  //      of the two-cell halo each (south, north, west, east)
+  const int rc = (ty + kHalo) * kReg + (tx + kHalo);
+  Q4<R> c = {R(0), R(0), R(0), R(0)};
+  uint8_t fown = 0;
   {
-    // U^n of the tile's own cells, which the update phase reads after the
-    // faces, into L1 now (FP64 step 0.798 -> 0.779 ms)
-    if (tid < 64) {
-      const int fld = tid >> 4;
-      const double *un = a.s0[fld == 0 ? F_RHO : (fld == 1 ? F_U : (fld == 2 ? F_V : F_E))];
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(un + (int64_t)tile * kTileCells + (tid & 15) * 16));
+    const int side = (NT >> 5) - 1 - (tid >> 5), i = tid & 31;
+    int64_t hs = -1;  // this lane's halo cell
+    int hr = 0;
+    if (side < 4) {
+      int x, y;  // position in the neighbour tile
+      if (side < 2) {
+        x = i & 15;
+        y = (side ? 0 : kTile - kHalo) + (i >> 4);
+        hr = ((i >> 4) + (side ? kTile + kHalo : 0)) * kReg + x + kHalo;
+      } else {
+        x = (side == 2 ? kTile - kHalo : 0) + (i & 1);
+        y = i >> 1;
+        hr = (y + kHalo) * kReg + (i & 1) + (side == 2 ? 0 : kTile + kHalo);
+      }
+      if (nb >= 0) hs = (int64_t)nb * kTileCells + y * kTile + x;
     }
-  }
-  if (prefetch > 0) {
-    // the CTA that starts when this one ends reads this tile's input from L2
-    constexpr int kLines = kTileCells * (int)sizeof(TI) / 128;  // 128-byte lines per field
-    const int64_t pt = (int64_t)(tile + prefetch) * kTileCells;
-    if (tid < 4 * kLines && pt < a.nslots)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const TI *>(v.sin[tid / kLines]) + pt +
-                                                    (tid % kLines) * (128 / (int)sizeof(TI))));
-  }
-
-  if (uni) {
-    // one region record per thread and pass: its four fields loaded (all
-    // loads of both passes issued before the first store), then one record
-    // store (no shared-memory bank conflicts); corners stay unset (a
-    // uniform tile's stencils never read them)
-    constexpr int NIT = (kReg * kReg + NT - 1) / NT;
+    const int64_t os = (int64_t)tile * kTileCells + (own ? tid : 0);
     const TI *in0 = static_cast<const TI *>(v.sin[0]), *in1 = static_cast<const TI *>(v.sin[1]),
              *in2 = static_cast<const TI *>(v.sin[2]), *in3 = static_cast<const TI *>(v.sin[3]);
-    R q[NIT][4];
-    bool has[NIT];
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int r = tid + it * NT;
-      const int rx = r % kReg - kHalo, ry = r / kReg - kHalo;
-      const int ox = rx < 0 ? -1 : (rx >= kTile ? 1 : 0);
-      const int oy = ry < 0 ? -1 : (ry >= kTile ? 1 : 0);
-      has[it] = r < kReg * kReg && !(ox && oy);
-      if (has[it]) {
-        const int nb = ox < 0 ? nbw : (ox > 0 ? nbe : (oy < 0 ? nbs : (oy > 0 ? nbn : tile)));
-        const int64_t sl = (int64_t)nb * kTileCells + (ry - oy * kTile) * kTile + (rx - ox * kTile);
-        q[it][0] = (R)__ldg(in0 + sl);
-        q[it][1] = (R)__ldg(in1 + sl);
-        q[it][2] = (R)__ldg(in2 + sl);
-        q[it][3] = (R)__ldg(in3 + sl);
+    Q4<R> h = {R(0), R(0), R(0), R(0)};
+    if (UNI) {
+      // every load before the first store
+      if (own) c = Q4<R>{(R)__ldg(in0 + os), (R)__ldg(in1 + os), (R)__ldg(in2 + os), (R)__ldg(in3 + os)};
+      if (side < 4) h = Q4<R>{(R)__ldg(in0 + hs), (R)__ldg(in1 + hs), (R)__ldg(in2 + hs), (R)__ldg(in3 + hs)};
+    } else {
+      // presence flags first, then the state of the present cells: the
+      // stage input where the stages write it, else the step state
+      uint8_t fh = 0;
+      if (own) fown = a.flags[os];
+      if (side < 4 && hs >= 0) fh = a.flags[hs];
+      if (fown & CF_PRESENT) {
+        if (fown & (CF_PRIM | CF_RESET))
+          c = Q4<R>{(R)in0[os], (R)in1[os], (R)in2[os], (R)in3[os]};
+        else
+          c = Q4<R>{(R)a.s0[F_RHO][os], (R)a.s0[F_U][os], (R)a.s0[F_V][os], (R)a.s0[F_P][os]};
       }
-    }
-#pragma unroll
-    for (int it = 0; it < NIT; ++it)
-      if (has[it]) S::st(sq, tid + it * NT, NQ, q[it][0], q[it][1], q[it][2], q[it][3]);
-  } else {
-    // region records: slot, then presence flags, then the state, each
-    // step's loads of both records issued together
-    constexpr int NIT = (kReg * kReg + NT - 1) / NT;
-    int64_t sl[NIT];
-    uint8_t fl[NIT];
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int r = tid + it * NT;
-      sl[it] = -1;
-      if (r < kReg * kReg) {
-        const int rx = r % kReg - kHalo, ry = r / kReg - kHalo;
-        const int ox = rx < 0 ? -1 : (rx >= kTile ? 1 : 0);
-        const int oy = ry < 0 ? -1 : (ry >= kTile ? 1 : 0);
-        if (!(ox && oy)) {
-          const int nb = ox < 0 ? nbw : (ox > 0 ? nbe : (oy < 0 ? nbs : (oy > 0 ? nbn : tile)));
-          if (nb >= 0) sl[it] = (int64_t)nb * kTileCells + (ry - oy * kTile) * kTile + (rx - ox * kTile);
-        }
+      if (fh & CF_PRESENT) {
+        if (fh & (CF_PRIM | CF_RESET))
+          h = Q4<R>{(R)in0[hs], (R)in1[hs], (R)in2[hs], (R)in3[hs]};
+        else
+          h = Q4<R>{(R)a.s0[F_RHO][hs], (R)a.s0[F_U][hs], (R)a.s0[F_V][hs], (R)a.s0[F_P][hs]};
       }
+      if (own) sfl[rc] = fown;
+      if (side < 4) sfl[hr] = fh;
     }
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) fl[it] = sl[it] >= 0 ? a.flags[sl[it]] : uint8_t(0);
-#pragma unroll
-    for (int it = 0; it < NIT; ++it) {
-      const int r = tid + it * NT;
-      if (r < kReg * kReg) {
-        R q0 = R(0), q1 = R(0), q2 = R(0), q3 = R(0);
-        if (fl[it] & CF_PRESENT) {
-          const int64_t s = sl[it];
-          const bool varying = (fl[it] & (CF_PRIM | CF_RESET)) != 0;
-          if (varying) {
-            q0 = (R) static_cast<const TI *>(v.sin[0])[s];
-            q1 = (R) static_cast<const TI *>(v.sin[1])[s];
-            q2 = (R) static_cast<const TI *>(v.sin[2])[s];
-            q3 = (R) static_cast<const TI *>(v.sin[3])[s];
-          } else {
-            q0 = (R)a.s0[F_RHO][s];
-            q1 = (R)a.s0[F_U][s];
-            q2 = (R)a.s0[F_V][s];
-            q3 = (R)a.s0[F_P][s];
-          }
-        }
-        sfl[r] = fl[it];
-        S::st(sq, r, NQ, q0, q1, q2, q3);
-      }
-    }
+    if (own) S::st(sq, rc, NQ, c.x, c.y, c.z, c.w);
+    if (side < 4) S::st(sq, hr, NQ, h.x, h.y, h.z, h.w);
   }
   __syncthreads();
 
-  // ---- per-cell limited slopes: (tx, ty) in both directions, then the
-  //      two outer columns (x) and rows (y) of the face stencils
-  if (NT > kTileCells) {
-    if (own) {
-      const int rc = (ty + kHalo) * kReg + (tx + kHalo);
-      fast_slope<R, LIM, NQ, NS>(sq, sfl, slx, ty * kSX + tx + 1, rc, 1, uni);
-      fast_slope<R, LIM, NQ, NS>(sq, sfl, sly, (ty + 1) * kTile + tx, rc, kReg, uni);
-    } else {
-      // ninth warp: one outer x-slope (columns -1, 16) and one outer
-      // y-slope (rows -1, 16) per lane
-      const int e = (tid - kTileCells) & 15, hi = (tid - kTileCells) >= 16;
-      const int col = hi ? kTile : -1;
-      fast_slope<R, LIM, NQ, NS>(sq, sfl, slx, e * kSX + col + 1, (e + kHalo) * kReg + col + kHalo,
-                                 1, uni);
-      const int row = hi ? kTile : -1;
-      fast_slope<R, LIM, NQ, NS>(sq, sfl, sly, (row + 1) * kTile + e,
-                                 (row + kHalo) * kReg + e + kHalo, kReg, uni);
-    }
-  } else {
-    const int rc = (ty + kHalo) * kReg + (tx + kHalo);
-    fast_slope<R, LIM, NQ, NS>(sq, sfl, slx, ty * kSX + tx + 1, rc, 1, uni);
-    fast_slope<R, LIM, NQ, NS>(sq, sfl, sly, (ty + 1) * kTile + tx, rc, kReg, uni);
-    if (tid < 64) {
-      const int e = tid & 15;
-      if (tid < 32) {
-        const int col = (tid < 16) ? -1 : kTile;
-        fast_slope<R, LIM, NQ, NS>(sq, sfl, slx, e * kSX + col + 1, (e + kHalo) * kReg + col + kHalo,
-                                   1, uni);
-      } else {
-        const int row = (tid < 48) ? -1 : kTile;
-        fast_slope<R, LIM, NQ, NS>(sq, sfl, sly, (row + 1) * kTile + e,
-                                   (row + kHalo) * kReg + e + kHalo, kReg, uni);
-      }
-    }
+  // ---- limited slopes and the cells' face states
+  Q4<R> wx = {}, wy = {}, we = {};  // own cell's state at its west / south face, edge cell's
+  if (own) {
+    Q4<R> hi;
+    cell_states<R, LIM, NQ>(sq, sfl, c, rc, 1, UNI, wx, hi);
+    S::st(fx, ty * kFX + tx + 1, NF, hi.x, hi.y, hi.z, hi.w);
+    cell_states<R, LIM, NQ>(sq, sfl, c, rc, kReg, UNI, wy, hi);
+    S::st(fy, (ty + 1) * kTile + tx, NF, hi.x, hi.y, hi.z, hi.w);
+  }
+  const bool xd = et < 16;  // edge lanes: east column, then north row
+  const int ee = et & 15, estep = xd ? 1 : kReg;
+  const int er = xd ? (ee + kHalo) * kReg + kTile + kHalo : (kTile + kHalo) * kReg + ee + kHalo;
+  if (et >= 0) {
+    // the cell before the first face of the row / column, and the one after
+    // its last face
+    const int r0 = er - (kTile + 1) * estep;
+    Q4<R> lo, hi;
+    cell_states<R, LIM, NQ>(sq, sfl, S::ld(sq, r0, NQ), r0, estep, UNI, lo, hi);
+    S::st(xd ? fx : fy, xd ? ee * kFX : ee, NF, hi.x, hi.y, hi.z, hi.w);
+    cell_states<R, LIM, NQ>(sq, sfl, S::ld(sq, er, NQ), er, estep, UNI, we, hi);
   }
   __syncthreads();
 
@@ -664,77 +578,64 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
   g.Ma = (R)cc.Ma;
   g.gm1 = (R)cc.gm1;
   g.gamaRg = (R)cc.gamaRg;
-  g.inv_Rg = (R)(1.0 / cc.Rg);
-  g.inv_gm1 = (R)(1.0 / cc.gm1);
-  g.gam_gm1 = (R)(cc.gama / cc.gm1);
-  g.two_gama = (R)(2.0 * cc.gama);
+  g.inv_Rg = (R)cc.inv_Rg;
+  g.gam_gm1 = (R)cc.gam_gm1;
+  g.two_gama = (R)cc.two_gama;
   const R ax = (R)L.area_x, ay = (R)L.area_y;
   const R hax = R(0.5) * ax, hay = R(0.5) * ay;
 
-  // ---- face fluxes: west x-face and south y-face of cell (tx, ty), plus the
-  //      east column (threads 0..15) and north row (threads 16..31)
-  {
-    const int rR1 = (ty + kHalo) * kReg + (tx + kHalo);
-    Q4<R> o;
-    if (!own) {
-      // ninth warp: edge faces only (below)
-    } else if constexpr (kPairFaces<R>) {
-      // the cell's west and south faces as the two lanes of one paired flux
-      // evaluation (f32x2 instructions in the mixed build)
-      R lx[4], rx[4], ly[4], ry[4];
-      const bool ax_ok = face_recon<R, LIM, NQ, NS>(sq, sfl, slx, rR1 - 1, rR1, 1, ty * kSX + tx,
-                                                   ty * kSX + tx + 1, uni, lx, rx);
-      const bool ay_ok = face_recon<R, LIM, NQ, NS>(sq, sfl, sly, rR1 - kReg, rR1, kReg,
-                                                   ty * kTile + tx, (ty + 1) * kTile + tx, uni, ly,
-                                                   ry);
+  // ---- face fluxes: west and south face of the own cell, then the edge
+  const Q4<R> none = {R(0), R(0), R(0), R(0)};
+  if (own) {
+    const int ix = ty * kFX + tx, iy = ty * kTile + tx;
+    const bool ax_ok = UNI || face_active(sfl[rc - 1], fown);
+    const bool ay_ok = UNI || face_active(sfl[rc - kReg], fown);
+    if constexpr (kPairFaces<R>) {
+      // both faces as the two lanes of one paired flux evaluation (f32x2
+      // instructions in the mixed build)
       using P = decltype(pair(R(0), R(0)));
+      const Q4<R> l = S::ld(fx, ix, NF), k = S::ld(fy, iy, NF);
       P fm, fn, ft, fe;
-      roe_flux_pair<P, R>(g, pair(ax, ay), pair(lx[0], ly[0]), pair(lx[1], ly[2]),
-                          pair(lx[2], ly[1]), pair(lx[3], ly[3]), pair(rx[0], ry[0]),
-                          pair(rx[1], ry[2]), pair(rx[2], ry[1]), pair(rx[3], ry[3]), fm, fn, ft,
-                          fe);
-      if (ax_ok) S::st(fx, ty * (kTile + 1) + tx, NF, lane0(fm), lane0(fn), lane0(ft), lane0(fe));
-      else S::st(fx, ty * (kTile + 1) + tx, NF, R(0), R(0), R(0), R(0));
-      if (ay_ok) S::st(fy, ty * kTile + tx, NF, lane1(fm), lane1(ft), lane1(fn), lane1(fe));
-      else S::st(fy, ty * kTile + tx, NF, R(0), R(0), R(0), R(0));
+      roe_flux_pair<P, R>(g, pair(ax, ay), pair(l.x, k.x), pair(l.y, k.z), pair(l.z, k.y),
+                          pair(l.w, k.w), pair(wx.x, wy.x), pair(wx.y, wy.z), pair(wx.z, wy.y),
+                          pair(wx.w, wy.w), fm, fn, ft, fe);
+      const Q4<R> fw = ax_ok ? Q4<R>{lane0(fm), lane0(fn), lane0(ft), lane0(fe)} : none;
+      const Q4<R> fs = ay_ok ? Q4<R>{lane1(fm), lane1(ft), lane1(fn), lane1(fe)} : none;
+      S::st(fx, ix, NF, fw.x, fw.y, fw.z, fw.w);
+      S::st(fy, iy, NF, fs.x, fs.y, fs.z, fs.w);
     } else {
-      o = fast_face<R, LIM, NQ, NS>(sq, sfl, slx, rR1 - 1, rR1, 1, ty * kSX + tx,
-                                    ty * kSX + tx + 1, true, uni, g, ax, hax);
-      S::st(fx, ty * (kTile + 1) + tx, NF, o.x, o.y, o.z, o.w);
-      o = fast_face<R, LIM, NQ, NS>(sq, sfl, sly, rR1 - kReg, rR1, kReg, ty * kTile + tx,
-                                    (ty + 1) * kTile + tx, false, uni, g, ay, hay);
-      S::st(fy, ty * kTile + tx, NF, o.x, o.y, o.z, o.w);
+      Q4<R> f = state_flux<R>(g, true, ax, hax, S::ld(fx, ix, NF), wx);
+      if (!ax_ok) f = none;
+      S::st(fx, ix, NF, f.x, f.y, f.z, f.w);
+      f = state_flux<R>(g, false, ay, hay, S::ld(fy, iy, NF), wy);
+      if (!ay_ok) f = none;
+      S::st(fy, iy, NF, f.x, f.y, f.z, f.w);
     }
-    const int et = tid - (NT > kTileCells ? kTileCells : 0);
-    if (et >= 0 && et < 32) {
-      // east column (lanes 0..15) and north row (lanes 16..31) through one
-      // call site, so the warp evaluates the flux once
-      const int e = et & 15;
-      const bool xd = et < 16;
-      const int r = xd ? (e + kHalo) * kReg + kTile + kHalo : (kTile + kHalo) * kReg + e + kHalo;
-      const int step = xd ? 1 : kReg;
-      const int sL = xd ? e * kSX + kTile : kTile * kTile + e;
-      const int sR = xd ? e * kSX + kTile + 1 : (kTile + 1) * kTile + e;
-      o = fast_face<R, LIM, NQ, NS>(sq, sfl, xd ? slx : sly, r - step, r, step, sL, sR, xd, uni,
-                                    g, xd ? ax : ay, xd ? hax : hay);
-      S::st(xd ? fx : fy, xd ? e * (kTile + 1) + kTile : kTile * kTile + e, NF, o.x, o.y, o.z, o.w);
-    }
+  }
+  if (et >= 0) {
+    // east column (lanes 0..15) and north row (lanes 16..31) through one
+    // call site, so the warp evaluates the flux once
+    V *fe = xd ? fx : fy;
+    const int k = xd ? ee * kFX + kTile : kTile * kTile + ee;
+    Q4<R> o = state_flux<R>(g, xd, xd ? ax : ay, xd ? hax : hay, S::ld(fe, k, NF), we);
+    if (!UNI && !face_active(sfl[er - estep], sfl[er])) o = none;
+    S::st(fe, k, NF, o.x, o.y, o.z, o.w);
   }
   __syncthreads();
 
   // ---- residual, update, primitive recovery (FP64)
   const int64_t slot = (int64_t)tile * kTileCells + tid;
   const uint8_t fl = !own ? (uint8_t)0
-                         : uni ? (uint8_t)(CF_PRESENT | CF_NORMAL | CF_UPDATE | CF_PRIM | CF_RESNORM)
-                               : sfl[(ty + kHalo) * kReg + (tx + kHalo)];
+                         : UNI ? (uint8_t)(CF_PRESENT | CF_NORMAL | CF_UPDATE | CF_PRIM | CF_RESNORM)
+                               : fown;
   unsigned long long rb[4] = {0ull, 0ull, 0ull, 0ull};
-  double cb = -1.0;  // next step's CFL bound of this cell, when this stage writes it
+  double cb = -1.0;  // the cell's sum for the next step's CFL bound, when this stage writes it
   if ((fl & CF_NORMAL) && (fl & (CF_UPDATE | CF_RESET))) {
-    const Q4<R> fxl = S::ld(fx, ty * (kTile + 1) + tx, NF), fxh = S::ld(fx, ty * (kTile + 1) + tx + 1, NF);
-    const Q4<R> fyl = S::ld(fy, ty * kTile + tx, NF), fyh = S::ld(fy, (ty + 1) * kTile + tx, NF);
+    const Q4<R> fw = S::ld(fx, ty * kFX + tx, NF), fxh = S::ld(fx, ty * kFX + tx + 1, NF);
+    const Q4<R> fs = S::ld(fy, ty * kTile + tx, NF), fyh = S::ld(fy, (ty + 1) * kTile + tx, NF);
     double res[4];
-    const R sxl[4] = {fxl.x, fxl.y, fxl.z, fxl.w}, sxh[4] = {fxh.x, fxh.y, fxh.z, fxh.w};
-    const R syl[4] = {fyl.x, fyl.y, fyl.z, fyl.w}, syh[4] = {fyh.x, fyh.y, fyh.z, fyh.w};
+    const R sxl[4] = {fw.x, fw.y, fw.z, fw.w}, sxh[4] = {fxh.x, fxh.y, fxh.z, fxh.w};
+    const R syl[4] = {fs.x, fs.y, fs.z, fs.w}, syh[4] = {fyh.x, fyh.y, fyh.z, fyh.w};
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       if (sizeof(R) == 4 && !VISC) {
@@ -805,20 +706,75 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
 #pragma unroll
       for (int c = 0; c < 4; ++c) rb[c] = (unsigned long long)__double_as_longlong(fabs(res[c]));
     }
-    if (FINAL && fold && wrote) cb = cfl_cell_bound(nT, nu, nv, L, cc);
+    if (FINAL && fold && wrote) cb = cfl_cell_sum(nT, nu, nv, L, cc);
   }
-  // the y-slope records are dead after the face phase: reuse them
+  // the region is dead after the face phase: reuse it
   if (FINAL) {
-    unsigned long long *sred = reinterpret_cast<unsigned long long *>(sly);
+    unsigned long long *sred = reinterpret_cast<unsigned long long *>(sq);
     block_resnorm<NT>(rb, a.diag, sred);
     if (fold) fold_next_cfl<NT>(a, L, cc, fl, slot, cb, sred, fold - 1, own);
   }
 }
 
+template <typename R, int LIM, bool VISC, bool FINAL, typename TI,
+          int NT = StageThreads<R>::value>
+__device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageVar &v,
+                                                const CaseConst &cc,
+                                                const int tile, const int phase,
+                                                const int fold, const int prefetch) {
+  using S = SRec<R>;
+  using V = typename S::V;
+  constexpr int kFX = kTile + 1;  // faces of a row
+  constexpr int NQ = kReg * kReg, NF = kTile * kFX;
+  __shared__ V sq[S::kPlanes * NQ];
+  __shared__ uint8_t sfl[NQ];
+  // face (i, j) between cells i-1 and i of row j at j*17 + i, between cells
+  // j-1 and j of column i at j*16 + i: the lower cell's state, then the flux
+  __shared__ V fx[S::kPlanes * NF];
+  __shared__ V fy[S::kPlanes * NF];
+
+  static_assert(NT == kTileCells || NT == kTileCells + 32, "256 or 288 threads");
+  const int tid = threadIdx.x;
+  const int lvl = a.tile_level[tile];
+  const LevelConst &L = cc.lev[lvl];
+  // uniform tile: it and its four side neighbours hold only leaf cells that
+  // recover their primitives, so no presence flags or one-sided stencils
+  const bool uni = a.tile_uniform != nullptr && a.tile_uniform[tile] != 0;
+
+  // this lane's side of the halo (south, north, west, east: four whole warps),
+  // looked up beside the tile's level and uniform flag, so that the region's
+  // loads wait for one round trip
+  const int side = (NT >> 5) - 1 - (tid >> 5);
+  const int nb = side < 4 ? __ldg(a.tile_nb + (int64_t)tile * 9 +
+                                  (side == 0 ? 1 : side == 1 ? 7 : side == 2 ? 3 : 5))
+                          : -1;
+
+  {
+    // U^n of the tile's own cells, which the update phase reads after the
+    // faces, into L1 now (FP64 step 0.798 -> 0.779 ms)
+    if (tid < 64) {
+      const int fld = tid >> 4;
+      const double *un = a.s0[fld == 0 ? F_RHO : (fld == 1 ? F_U : (fld == 2 ? F_V : F_E))];
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(un + (int64_t)tile * kTileCells + (tid & 15) * 16));
+    }
+  }
+  if (prefetch > 0) {
+    // the CTA that starts when this one ends reads this tile's input from L2
+    constexpr int kLines = kTileCells * (int)sizeof(TI) / 128;  // 128-byte lines per field
+    const int64_t pt = (int64_t)(tile + prefetch) * kTileCells;
+    if (tid < 4 * kLines && pt < a.nslots)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const TI *>(v.sin[tid / kLines]) + pt +
+                                                    (tid % kLines) * (128 / (int)sizeof(TI))));
+  }
+
+  if (uni) stage_tile<R, LIM, VISC, FINAL, TI, NT, true>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
+  else stage_tile<R, LIM, VISC, FINAL, TI, NT, false>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
+}
+
 // TI: element type of the stage input (the FP64 step state for the first
 // stage; the stage buffers, R, after it)
 template <typename R, int LIM, bool VISC, bool FINAL, typename TI>
-__global__ void __launch_bounds__(StageThreads<R>::value, sizeof(R) == 8 ? 4 : 6)
+__global__ void __launch_bounds__(StageThreads<R>::value, stage_min_blocks<R, StageThreads<R>::value>())
     stage_kernel_fast(StageArgs a, CaseConst cc) {
   stage_tile_fast<R, LIM, VISC, FINAL, TI>(a, a.v, cc, a.tile_begin + blockIdx.x, a.phase,
                                            a.v.cfl_next, a.prefetch);

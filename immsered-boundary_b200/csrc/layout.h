@@ -45,6 +45,7 @@ struct LevelConst {
 struct CaseConst {
   double gama, Rg, Cv, Ma, Re, qk, s_over_t, dt_ratio;
   double gm1, gamaRg, inv_Rg, Cp;
+  double gam_gm1, two_gama;  // gama / (gama - 1), 2 gama (fast builds)
   double p_ref, area_ref, shear_ref, L_ref, mu;
   double initvar[7];
   LevelConst lev[kMaxLevels];
