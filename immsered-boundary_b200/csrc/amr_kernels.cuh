@@ -16,13 +16,18 @@ namespace IBGPU_KNS {
 // (AMRInterface.cpp:78-110, TwoLevelOp.H:67-87, 225-231): density-weighted
 // mean of the four sons written to the coarse ghost.
 __global__ void restrict_kernel(PairArgs a, CaseConst cc) {
+  dep_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   double *const *q = a.s0;
   double roe = 0.0, u = 0.0, v = 0.0, e = 0.0;
+  const int4 fine = reinterpret_cast<const int4 *>(a.fine)[i];
+  const int sons[4] = {fine.x, fine.y, fine.z, fine.w};
+  const int c = a.coarse[i];
+  dep_wait();
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    int f = a.fine[4 * i + k];
+    int f = sons[k];
     double r = q[F_RHO][f];
     roe += r;
     u += q[F_U][f] * r;
@@ -35,7 +40,6 @@ __global__ void restrict_kernel(PairArgs a, CaseConst cc) {
   roe *= 0.25;
   double p = (e - 0.5 * (u * u + v * v)) * cc.gm1 * roe;
   double T = p / (roe * cc.Rg);
-  int c = a.coarse[i];
   q[F_RHO][c] = roe;
   q[F_U][c] = u;
   q[F_V][c] = v;
@@ -49,12 +53,17 @@ __global__ void restrict_kernel(PairArgs a, CaseConst cc) {
 // neighbours, central gradients (q+ - q-)/2, sons at offsets -/+ 1/4,
 // primitive recovery of each son.
 __global__ void prolong_kernel(PairArgs a, CaseConst cc) {
+  dep_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   double *const *q = a.s0;
   // neighbour order: -x, +x, -y, +y
   double U[5][4];
-  int cells[5] = {a.coarse[i], a.nb[4 * i + 0], a.nb[4 * i + 1], a.nb[4 * i + 2], a.nb[4 * i + 3]};
+  const int4 nb = reinterpret_cast<const int4 *>(a.nb)[i];
+  const int4 fine = reinterpret_cast<const int4 *>(a.fine)[i];
+  const int cells[5] = {a.coarse[i], nb.x, nb.y, nb.z, nb.w};
+  const int sons[4] = {fine.x, fine.y, fine.z, fine.w};
+  dep_wait();
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     int s = cells[k];
@@ -84,7 +93,7 @@ __global__ void prolong_kernel(PairArgs a, CaseConst cc) {
       double e = f[3] / f[0];
       double p = (e - 0.5 * (u * u + vv * vv)) * cc.gm1 * roe;
       double T = p / (roe * cc.Rg);
-      int s = a.fine[4 * i + si * 2 + sj];
+      int s = sons[si * 2 + sj];
       q[F_RHO][s] = roe;
       q[F_U][s] = u;
       q[F_V][s] = vv;
@@ -96,12 +105,14 @@ __global__ void prolong_kernel(PairArgs a, CaseConst cc) {
 
 // ---- domain boundary ghosts (BCValues::BCBoxTreat, BCValues.H:51-298) ----
 __global__ void bc_kernel(BcArgs a, CaseConst cc) {
+  dep_begin();
   int i = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.end) return;
   double *const *q = a.s0;
   const int g = a.ghost[i], r = a.ref[i];
   const int type = a.type[i];
   const double *fv = a.facevar + 7 * a.face[i];
+  dep_wait();
   double roe = q[F_RHO][r], u = q[F_U][r], v = q[F_V][r], p = q[F_P][r], T = q[F_T][r],
          e = q[F_E][r];
   switch (type) {
@@ -185,11 +196,9 @@ __device__ __forceinline__ void image_point(const int32_t *cells, const double *
   roe = p / (cc.Rg * T);
 }
 
-// Phase 1: every IB cell's new state from the current field (the reference
-// computes them all before writing any, Body.cpp:1361-1488).
-__global__ void ib_compute_kernel(IbArgs a, CaseConst cc) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+// New state of IB cell i (rho u v p e T) from the current field.
+__device__ __forceinline__ void ib_cell(const IbArgs &a, const CaseConst &cc, int i,
+                                        double (&o)[6]) {
   const double *f = a.cellf + 16 * i;  // signdis, hgdis, w[8], nv[3], patv[3]
   double hT, hp, hu, hv, hroe;
   image_point(a.intp + 8 * i, f + 2, a.s0, cc, hT, hp, hu, hv, hroe);
@@ -214,7 +223,6 @@ __global__ void ib_compute_kernel(IbArgs a, CaseConst cc) {
   }
   double roe = p / (cc.Rg * T);
   double e = cc.Cv * T + 0.5 * (u * u + v * v + w * w);
-  double *o = a.out + 6 * i;
   o[0] = roe;
   o[1] = u;
   o[2] = v;
@@ -227,18 +235,47 @@ __global__ void ib_compute_kernel(IbArgs a, CaseConst cc) {
     raise_error(a.diag, phase, ERR_IB_NAN, a.cell[i]);
 }
 
-// Phase 2: write them (Body.cpp:1490-1494)
-__global__ void ib_store_kernel(IbArgs a) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const double *o = a.out + 6 * i;
-  int s = a.cell[i];
+__device__ __forceinline__ void ib_put(const IbArgs &a, int i, const double (&o)[6]) {
+  const int s = a.cell[i];
   a.s0[F_RHO][s] = o[0];
   a.s0[F_U][s] = o[1];
   a.s0[F_V][s] = o[2];
   a.s0[F_P][s] = o[3];
   a.s0[F_E][s] = o[4];
   a.s0[F_T][s] = o[5];
+}
+
+// The reference computes every IB cell's state before it writes any
+// (Body.cpp:1361-1494).  Up to kIbBlock cells: one CTA, a barrier between the
+// two halves (the airfoils have a few hundred cells: one launch instead of
+// two).  More: two launches with the states in between in a.out.
+constexpr int kIbBlock = 1024;
+__global__ void __launch_bounds__(kIbBlock) ib_kernel(IbArgs a, CaseConst cc) {
+  dep_begin();
+  dep_wait();
+  const int i = threadIdx.x;
+  double o[6];
+  if (i < a.n) ib_cell(a, cc, i, o);
+  __syncthreads();
+  if (i < a.n) ib_put(a, i, o);
+}
+__global__ void ib_compute_kernel(IbArgs a, CaseConst cc) {
+  dep_begin();
+  dep_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  double o[6];
+  ib_cell(a, cc, i, o);
+  for (int k = 0; k < 6; ++k) a.out[6 * i + k] = o[k];
+}
+__global__ void ib_store_kernel(IbArgs a) {
+  dep_begin();
+  dep_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  double o[6];
+  for (int k = 0; k < 6; ++k) o[k] = a.out[6 * i + k];
+  ib_put(a, i, o);
 }
 
 // ---- wall forces (Body::ComptWallForce, Body.cpp:439-558) ----------------
@@ -332,6 +369,8 @@ __global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseCon
   const int tid = threadIdx.x;
   const int tile = a.tile_begin + blockIdx.x;
   const LevelConst &L = cc.lev[a.tile_level[tile]];
+  dep_begin();
+  dep_wait();
   for (int r = tid; r < G * G; r += kTileCells) {
     int rx = r % G - H, ry = r / G - H;
     int ox = rx < 0 ? -1 : (rx >= kTile ? 1 : 0);
@@ -437,35 +476,39 @@ __global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseCon
 }
 
 // ---- launchers ---------------------------------------------------------------
-void launch_restrict(const PairArgs &a, const CaseConst &cc, cudaStream_t st) {
-  if (a.n > 0) restrict_kernel<<<(a.n + 127) / 128, 128, 0, st>>>(a, cc);
+void launch_restrict(const PairArgs &a, const CaseConst &cc, cudaStream_t st, bool dep) {
+  if (a.n > 0) launch_dep(dep, st, (a.n + 127) / 128, 128, restrict_kernel, a, cc);
 }
-void launch_prolong(const PairArgs &a, const CaseConst &cc, cudaStream_t st) {
-  if (a.n > 0) prolong_kernel<<<(a.n + 127) / 128, 128, 0, st>>>(a, cc);
+void launch_prolong(const PairArgs &a, const CaseConst &cc, cudaStream_t st, bool dep) {
+  if (a.n > 0) launch_dep(dep, st, (a.n + 127) / 128, 128, prolong_kernel, a, cc);
 }
-void launch_bc(const BcArgs &a, const CaseConst &cc, cudaStream_t st) {
+void launch_bc(const BcArgs &a, const CaseConst &cc, cudaStream_t st, bool dep) {
   int n = a.end - a.begin;
-  if (n > 0) bc_kernel<<<(n + 127) / 128, 128, 0, st>>>(a, cc);
+  if (n > 0) launch_dep(dep, st, (n + 127) / 128, 128, bc_kernel, a, cc);
 }
-void launch_ib(const IbArgs &a, const CaseConst &cc, cudaStream_t st) {
+void launch_ib(const IbArgs &a, const CaseConst &cc, cudaStream_t st, bool dep) {
   if (a.n <= 0) return;
-  ib_compute_kernel<<<(a.n + 127) / 128, 128, 0, st>>>(a, cc);
-  ib_store_kernel<<<(a.n + 127) / 128, 128, 0, st>>>(a);
+  if (a.n <= kIbBlock) {
+    launch_dep(dep, st, 1, (a.n + 31) / 32 * 32, ib_kernel, a, cc);
+    return;
+  }
+  launch_dep(dep, st, (a.n + 127) / 128, 128, ib_compute_kernel, a, cc);
+  launch_dep(true, st, (a.n + 127) / 128, 128, ib_store_kernel, a);
 }
 void launch_forces(const ForceArgs &a, const CaseConst &cc, cudaStream_t st) {
   if (a.n > 0) patch_force_kernel<<<(a.n + 127) / 128, 128, 0, st>>>(a, cc);
   force_sum_kernel<<<1, 256, 0, st>>>(a, cc);
 }
 void launch_viscous(const ViscArgs &a, const CaseConst &cc, int ntiles, bool mixed,
-                    cudaStream_t st) {
+                    cudaStream_t st, bool dep) {
   if (ntiles <= 0) return;
 #ifdef IBGPU_FAST_BUILD
   if (mixed) {
-    viscous_kernel<float><<<ntiles, kTileCells, 0, st>>>(a, cc);
+    launch_dep(dep, st, ntiles, kTileCells, viscous_kernel<float>, a, cc);
     return;
   }
 #endif
-  viscous_kernel<double><<<ntiles, kTileCells, 0, st>>>(a, cc);
+  launch_dep(dep, st, ntiles, kTileCells, viscous_kernel<double>, a, cc);
 }
 
 }  // namespace IBGPU_KNS

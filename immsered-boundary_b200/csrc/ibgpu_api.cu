@@ -10,6 +10,7 @@
 #include <new>
 #include <string>
 #include <unordered_map>
+#include <unordered_set>
 #include <map>
 #include <numeric>
 #include <vector>
@@ -122,12 +123,22 @@ struct ibgpu_ctx {
   // slot lookup: per level, tile (tx,ty) -> tile index
   std::vector<std::unordered_map<uint64_t, int>> tilemap;
 
-  // coarse/fine pairs per coarse level
+  // coarse/fine pairs: every level's in one list, coarse levels ascending;
+  // level l's are [begin[l], begin[l+1]).  joins[l]: level l's pairs may run
+  // together with level l-1's (they read nothing that those write).
   struct DevPairs {
     int32_t *coarse = nullptr, *fine = nullptr, *nb = nullptr;
-    int n = 0;
+    std::vector<int> begin;
+    std::vector<char> joins;
+    int count(int l) const { return l + 1 < (int)begin.size() ? begin[l + 1] - begin[l] : 0; }
+    void free() {
+      cudaFree(coarse);
+      cudaFree(fine);
+      cudaFree(nb);
+      *this = DevPairs();
+    }
   };
-  std::vector<DevPairs> res, pro;
+  DevPairs res, pro;
 
   // domain ghosts: level-sorted, dependency waves [begin, end)
   int32_t *d_bc_ghost = nullptr, *d_bc_ref = nullptr, *d_bc_type = nullptr, *d_bc_face = nullptr;
@@ -152,14 +163,8 @@ struct ibgpu_ctx {
   int64_t klaunch[3] = {0, 0, 0};
 
   void free_aux() {
-    for (auto *v : {&res, &pro})
-      for (auto &p : *v) {
-        cudaFree(p.coarse);
-        cudaFree(p.fine);
-        cudaFree(p.nb);
-      }
-    res.clear();
-    pro.clear();
+    res.free();
+    pro.free();
     for (int32_t **p : {&d_bc_ghost, &d_bc_ref, &d_bc_type, &d_bc_face, &d_ib_cell, &d_ib_intp,
                         &d_pat_body, &d_pat_intp, &d_body_begin}) {
       cudaFree(*p);
@@ -1038,11 +1043,43 @@ bool folds_cfl(const ibgpu_ctx *ctx) {
          ctx->cs.dt_var_step == 1;
 }
 
+// Runs of consecutive levels [l0, l1) below nlev that `on` holds for and
+// that may run together: f(l0, l1) for each.
+extern "C++" template <typename On, typename Join, typename F>
+int level_runs(int nlev, On on, Join joins, F f) {
+  for (int l = 0; l < nlev;) {
+    if (!on(l)) {
+      ++l;
+      continue;
+    }
+    int e = l + 1;
+    while (e < nlev && on(e) && joins(e)) ++e;
+    const int rc = f(l, e);
+    if (rc) return rc;
+    l = e;
+  }
+  return IBGPU_OK;
+}
+
+// Whether the first stage of step ts resets the step's reductions itself.
+// It does not when it is the final one (which accumulates them) or no level
+// marches at ts.
+bool stage_resets(const ibgpu_ctx *ctx, int ts) {
+  const ibgpu_case &cs = ctx->cs;
+  bool any = false;
+  for (int l = 0; l < cs.nlevels; ++l)
+    any = any || (ts % cs.march_step[l] == cs.march_left[l] && ctx->level_tile_count[l] > 0);
+  return any && cs.nstages > 1;
+}
+
 // Everything of step ts before the stages (main.cpp:87-89 and the frozen
-// part of NS_Solver::TimeMarching): reduction reset, restriction and
-// prolongation on their schedules, immersed-body ghosts, CFL dt, domain
-// ghosts and the viscous flux of the levels that march.
-int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer &tm,
+// part of NS_Solver::TimeMarching): restriction and prolongation on their
+// schedules, immersed-body ghosts, CFL dt, domain ghosts and the viscous flux
+// of the levels that march.  Levels that run together share a launch: their
+// tiles and pairs lie one after another, and a 24-tile level by itself leaves
+// most of the chip idle for its launch.  dep: whether the next launch may
+// overlap its predecessor's end (false for the first of a run).
+int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer &tm, bool &dep,
                      bool batched = false, bool fresh_cfl = false,
                      const int *phase_base = nullptr) {
   const ibgpu_case &cs = ctx->cs;
@@ -1052,35 +1089,40 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
   // a batch resets the reductions and runs the CFL pass of all its cases in
   // merged launches (the CFL pass reads normal cells only, which the domain
   // ghosts and the viscous pass below do not write, so it may follow them)
-  if (step > 0 && !batched) {
-    if (exact) exact::launch_step_begin(ctx->d_diag, st);
-    else fast::launch_step_begin(ctx->d_diag, st);
+  if (step > 0 && !batched && !stage_resets(ctx, ts)) {
+    if (exact) exact::launch_step_begin(ctx->d_diag, st, dep);
+    else fast::launch_step_begin(ctx->d_diag, st, dep);
+    dep = true;
   }
   // AMR::InterfaceExchange (AMRInterface.cpp:3-35): restriction of every
   // scheduled pair (coarse level ascending), then prolongation
-  for (int l = 0; l + 1 < cs.nlevels && l < (int)ctx->res.size(); ++l) {
-    if (ts % cs.average_step[l + 1] != cs.average_left[l + 1] || ctx->res[l].n == 0) continue;
-    PairArgs pa;
-    pa.coarse = ctx->res[l].coarse;
-    pa.fine = ctx->res[l].fine;
-    pa.nb = nullptr;
-    pa.n = ctx->res[l].n;
-    for (int f = 0; f < kStateFields; ++f) pa.s0[f] = ctx->d_s0[f];
-    if (exact) exact::launch_restrict(pa, ctx->cc, st);
-    else fast::launch_restrict(pa, ctx->cc, st);
-    CK(cudaGetLastError());
-  }
-  for (int l = 0; l + 1 < cs.nlevels && l < (int)ctx->pro.size(); ++l) {
-    if (ts % cs.prolong_step[l + 1] != cs.prolong_left[l + 1] || ctx->pro[l].n == 0) continue;
-    PairArgs pa;
-    pa.coarse = ctx->pro[l].coarse;
-    pa.fine = ctx->pro[l].fine;
-    pa.nb = ctx->pro[l].nb;
-    pa.n = ctx->pro[l].n;
-    for (int f = 0; f < kStateFields; ++f) pa.s0[f] = ctx->d_s0[f];
-    if (exact) exact::launch_prolong(pa, ctx->cc, st);
-    else fast::launch_prolong(pa, ctx->cc, st);
-    CK(cudaGetLastError());
+  for (int pass = 0; pass < 2; ++pass) {
+    const ibgpu_ctx::DevPairs &P = pass ? ctx->pro : ctx->res;
+    const int *every = pass ? cs.prolong_step : cs.average_step;
+    const int *left = pass ? cs.prolong_left : cs.average_left;
+    const int rc = level_runs(
+        cs.nlevels - 1,
+        [&](int l) { return ts % every[l + 1] == left[l + 1] && P.count(l) > 0; },
+        [&](int l) { return P.joins[l] != 0; },
+        [&](int l0, int l1) {
+          PairArgs pa;
+          pa.coarse = P.coarse + P.begin[l0];
+          pa.fine = P.fine + 4 * (size_t)P.begin[l0];
+          pa.nb = pass ? P.nb + 4 * (size_t)P.begin[l0] : nullptr;
+          pa.n = P.begin[l1] - P.begin[l0];
+          for (int f = 0; f < kStateFields; ++f) pa.s0[f] = ctx->d_s0[f];
+          if (pass) {
+            if (exact) exact::launch_prolong(pa, ctx->cc, st, dep);
+            else fast::launch_prolong(pa, ctx->cc, st, dep);
+          } else {
+            if (exact) exact::launch_restrict(pa, ctx->cc, st, dep);
+            else fast::launch_restrict(pa, ctx->cc, st, dep);
+          }
+          dep = true;
+          CK(cudaGetLastError());
+          return (int)IBGPU_OK;
+        });
+    if (rc) return rc;
   }
   // Body::IBConditions_Image (static bodies): IB ghost cells of the finest level
   if (ctx->n_ib > 0) {
@@ -1096,8 +1138,9 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
     ia.phase = phase_base ? 0 : pbase + 0;
     ia.phase_base = phase_base;
     ia.diag = ctx->d_diag;
-    if (exact) exact::launch_ib(ia, ctx->cc, st);
-    else fast::launch_ib(ia, ctx->cc, st);
+    if (exact) exact::launch_ib(ia, ctx->cc, st, dep);
+    else fast::launch_ib(ia, ctx->cc, st, dep);
+    dep = true;
     CK(cudaGetLastError());
   }
 
@@ -1106,8 +1149,9 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
   // previous step already accumulated the bound
   if (!batched && (ts % cs.dt_var_step) == 0 && step > 0 && !fresh_cfl && folds_cfl(ctx)) {
     cudaEvent_t e = tm.mark(2);
-    if (exact) exact::launch_take_folded_cfl(ctx->d_diag, ctx->cc, st);
-    else fast::launch_take_folded_cfl(ctx->d_diag, ctx->cc, st);
+    if (exact) exact::launch_take_folded_cfl(ctx->d_diag, ctx->cc, st, dep);
+    else fast::launch_take_folded_cfl(ctx->d_diag, ctx->cc, st, dep);
+    dep = true;
     tm.done(e);
     CK(cudaGetLastError());
   } else if (!batched && (ts % cs.dt_var_step) == 0) {
@@ -1119,8 +1163,9 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
     ca.phase = pbase + 1;
     ca.diag = ctx->d_diag;
     cudaEvent_t e = tm.mark(2);
-    if (exact) exact::launch_cfl(ca, ctx->cc, ctx->nsm, st);
-    else fast::launch_cfl(ca, ctx->cc, ctx->nsm, st);
+    if (exact) exact::launch_cfl(ca, ctx->cc, ctx->nsm, st, dep);
+    else fast::launch_cfl(ca, ctx->cc, ctx->nsm, st, dep);
+    dep = true;
     tm.done(e);
     CK(cudaGetLastError());
   }
@@ -1142,8 +1187,9 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
       ba.cos_in = ctx->cos_in;
       ba.sin_in = ctx->sin_in;
       for (int f = 0; f < kStateFields; ++f) ba.s0[f] = ctx->d_s0[f];
-      if (exact) exact::launch_bc(ba, ctx->cc, st);
-      else fast::launch_bc(ba, ctx->cc, st);
+      if (exact) exact::launch_bc(ba, ctx->cc, st, dep);
+      else fast::launch_bc(ba, ctx->cc, st, dep);
+      dep = true;
       CK(cudaGetLastError());
     }
   }
@@ -1156,15 +1202,22 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
     for (int f = 0; f < kStateFields; ++f) va.s0[f] = ctx->d_s0[f];
     va.vsd = ctx->d_vsd;
     va.nslots = ctx->nslots;
-    for (int l = 0; l < cs.nlevels; ++l) {
-      if (ts % cs.march_step[l] != cs.march_left[l]) continue;
-      va.tile_begin = ctx->level_tile_begin[l];
-      cudaEvent_t e = tm.mark(1);
-      if (exact) exact::launch_viscous(va, ctx->cc, ctx->level_tile_count[l], false, st);
-      else fast::launch_viscous(va, ctx->cc, ctx->level_tile_count[l], mixed, st);
-      tm.done(e);
-      CK(cudaGetLastError());
-    }
+    const int rc = level_runs(
+        cs.nlevels, [&](int l) { return ts % cs.march_step[l] == cs.march_left[l]; },
+        [](int) { return true; },
+        [&](int l0, int l1) {
+          va.tile_begin = ctx->level_tile_begin[l0];
+          const int nt = ctx->level_tile_begin[l1 - 1] + ctx->level_tile_count[l1 - 1] - va.tile_begin;
+          if (nt <= 0) return (int)IBGPU_OK;
+          cudaEvent_t e = tm.mark(1);
+          if (exact) exact::launch_viscous(va, ctx->cc, nt, false, st, dep);
+          else fast::launch_viscous(va, ctx->cc, nt, mixed, st, dep);
+          dep = true;
+          tm.done(e);
+          CK(cudaGetLastError());
+          return (int)IBGPU_OK;
+        });
+    if (rc) return rc;
   }
   return IBGPU_OK;
 }
@@ -1257,7 +1310,7 @@ constexpr int kMaxChainSteps = 1 << 20;
 // the tiles of the levels that march at ts; fold_next: the final stage
 // accumulates the next step's CFL bound where the case allows it.
 static int enqueue_stages(ibgpu_ctx *ctx, int ts, int step, bool fold_next, cudaStream_t st,
-                          RunTimer &tm) {
+                          RunTimer &tm, bool &dep) {
   const ibgpu_case &cs = ctx->cs;
   const bool exact = cs.precision == IBGPU_FP64_EXACT;
   const bool mixed = cs.precision == IBGPU_MIXED;
@@ -1267,15 +1320,25 @@ static int enqueue_stages(ibgpu_ctx *ctx, int ts, int step, bool fold_next, cuda
     sa.phase = 8 * step + 2 + k;
     const bool fin = (k == cs.nstages - 1);
     if (fin && fold_next && folds_cfl(ctx)) sa.v.cfl_next = 1 + 8 * (step + 1) + 1;
-    for (int l = 0; l < cs.nlevels; ++l) {
-      if (ts % cs.march_step[l] != cs.march_left[l]) continue;
-      sa.tile_begin = ctx->level_tile_begin[l];
-      cudaEvent_t e = tm.mark(0);
-      if (exact) exact::launch_stage(sa, ctx->cc, ctx->level_tile_count[l], cs.limiter, cs.viscous != 0, fin, false, k, st);
-      else fast::launch_stage(sa, ctx->cc, ctx->level_tile_count[l], cs.limiter, cs.viscous != 0, fin, mixed, k, st);
-      tm.done(e);
-      CK(cudaGetLastError());
-    }
+    if (k == 0 && step > 0 && stage_resets(ctx, ts))
+      sa.reset = 1 | (ts % cs.dt_var_step != 0 ? 2 : 0);
+    const int rc = level_runs(
+        cs.nlevels, [&](int l) { return ts % cs.march_step[l] == cs.march_left[l]; },
+        [](int) { return true; },
+        [&](int l0, int l1) {
+          sa.tile_begin = ctx->level_tile_begin[l0];
+          const int nt = ctx->level_tile_begin[l1 - 1] + ctx->level_tile_count[l1 - 1] - sa.tile_begin;
+          if (nt <= 0) return (int)IBGPU_OK;
+          cudaEvent_t e = tm.mark(0);
+          if (exact) exact::launch_stage(sa, ctx->cc, nt, cs.limiter, cs.viscous != 0, fin, false, k, st, dep);
+          else fast::launch_stage(sa, ctx->cc, nt, cs.limiter, cs.viscous != 0, fin, mixed, k, st, dep);
+          dep = true;
+          sa.reset = 0;  // once per step
+          tm.done(e);
+          CK(cudaGetLastError());
+          return (int)IBGPU_OK;
+        });
+    if (rc) return rc;
   }
   return IBGPU_OK;
 }
@@ -1293,11 +1356,12 @@ static int run_steps(ibgpu_ctx *ctx, int ts0, int nsteps, double *dt, ibgpu_diag
   if ((rc = begin_diag(ctx, *dt, st))) return rc;
   RunTimer tm{ctx, st, {}, {}};
   int64_t marched = 0;
+  bool dep = false;
   for (int step = 0; step < nsteps; ++step) {
     const int ts = ts0 + step;
-    if ((rc = enqueue_prestage(ctx, ts, step, st, tm))) return rc;
+    if ((rc = enqueue_prestage(ctx, ts, step, st, tm, dep))) return rc;
     marched = marched_cells(ctx, ts);
-    if ((rc = enqueue_stages(ctx, ts, step, step + 1 < nsteps, st, tm))) return rc;
+    if ((rc = enqueue_stages(ctx, ts, step, step + 1 < nsteps, st, tm, dep))) return rc;
   }
   CK(cudaMemcpyAsync(ctx->h_diag, ctx->d_diag, sizeof(DevDiag), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -1358,8 +1422,9 @@ int ibgpu_step_async(ibgpu_ctx *ctx, int ts, double dt) {
   // a fresh CFL pass every step (the state may have been replaced since the
   // previous one), so no fold into the final stage either
   const int step = ctx->chain_steps;
-  if ((rc = enqueue_prestage(ctx, ts, step, st, tm, false, true))) return rc;
-  if ((rc = enqueue_stages(ctx, ts, step, false, st, tm))) return rc;
+  bool dep = false;  // what came before may be an upload's scatter
+  if ((rc = enqueue_prestage(ctx, ts, step, st, tm, dep, false, true))) return rc;
+  if ((rc = enqueue_stages(ctx, ts, step, false, st, tm, dep))) return rc;
   ctx->chain_marched = marched_cells(ctx, ts);
   ctx->chain_steps = step + 1;
   return IBGPU_OK;
@@ -1631,7 +1696,8 @@ int batch_step_graph(ibgpu_batch *b, int q, int cfl, cudaGraphExec_t *out) {
   for (size_t i = 0; i < b->cases.size() && e == cudaSuccess && !rc; ++i) {
     RunTimer tm{b->cases[i], b->fork[i % nf], {}, {}};
     tm.off = true;
-    rc = enqueue_prestage(b->cases[i], q, 1, b->fork[i % nf], tm, true, false, b->d_phase_base);
+    bool dep = false;
+    rc = enqueue_prestage(b->cases[i], q, 1, b->fork[i % nf], tm, dep, true, false, b->d_phase_base);
   }
   for (int k = 0; k < nf && e == cudaSuccess && !rc; ++k) {
     e = cudaEventRecord(b->ev_fork_join[k], b->fork[k]);
@@ -1893,8 +1959,10 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
       if ((rc = batch_step_graph(b, ts % b->full_period, cfl, &gx))) return rc;
       CK(cudaGraphLaunch(gx, st));
     } else {
-      for (int i = 0; i < n; ++i)
-        if ((rc = enqueue_prestage(b->cases[i], ts, step, st, tms[i], true))) return rc;
+      for (int i = 0; i < n; ++i) {
+        bool dep = false;
+        if ((rc = enqueue_prestage(b->cases[i], ts, step, st, tms[i], dep, true))) return rc;
+      }
       if (b->timing) {
         CK(cudaEventCreate(&e0));
         CK(cudaEventCreate(&e1));
@@ -2063,14 +2131,8 @@ int ibgpu_upload_interfaces(ibgpu_ctx *ctx, const ibgpu_cf_pairs *pp) {
   const int nlev = ctx->cs.nlevels;
   cudaStream_t st = ctx->stream;
   CK(cudaStreamSynchronize(st));
-  for (auto *v : {&ctx->res, &ctx->pro})
-    for (auto &p : *v) {
-      cudaFree(p.coarse);
-      cudaFree(p.fine);
-      cudaFree(p.nb);
-    }
-  ctx->res.assign(nlev, {});
-  ctx->pro.assign(nlev, {});
+  ctx->res.free();
+  ctx->pro.free();
   // restriction: per coarse level, in list order
   std::vector<std::vector<int32_t>> rc_(nlev), rf(nlev);
   for (int64_t i = 0; i < pp->nres; ++i) {
@@ -2118,15 +2180,40 @@ int ibgpu_upload_interfaces(ibgpu_ctx *ctx, const ibgpu_cf_pairs *pp) {
     pc[l].push_back((int32_t)c);
     for (int k = 0; k < 4; ++k) pf[l].push_back((int32_t)sons[k]);
   }
-  int e;
-  for (int l = 0; l < nlev; ++l) {
-    if ((e = upload_vec(&ctx->res[l].coarse, rc_[l], st)) || (e = upload_vec(&ctx->res[l].fine, rf[l], st)) ||
-        (e = upload_vec(&ctx->pro[l].coarse, pc[l], st)) || (e = upload_vec(&ctx->pro[l].fine, pf[l], st)) ||
-        (e = upload_vec(&ctx->pro[l].nb, pn[l], st)))
+  // all levels in one list each; a level joins the one before it when it
+  // reads no slot that the other writes (and, restricting, writes none that
+  // the other reads), so that the order between them does not matter
+  auto pack = [&](ibgpu_ctx::DevPairs &P, const std::vector<std::vector<int32_t>> &c,
+                  const std::vector<std::vector<int32_t>> &f,
+                  const std::vector<std::vector<int32_t>> *nb) -> int {
+    std::vector<int32_t> ac, af, an;
+    P.begin.assign(nlev + 1, 0);
+    P.joins.assign(nlev, 0);
+    for (int l = 0; l < nlev; ++l) {
+      P.begin[l] = (int)ac.size();
+      if (l > 0) {
+        const std::vector<int32_t> &wrote = nb ? f[l - 1] : c[l], &a1 = nb ? c[l] : f[l - 1];
+        std::unordered_set<int32_t> w(wrote.begin(), wrote.end());
+        bool free = true;
+        for (int32_t x : a1) free = free && !w.count(x);
+        if (nb)
+          for (int32_t x : (*nb)[l]) free = free && !w.count(x);
+        P.joins[l] = free;
+      }
+      ac.insert(ac.end(), c[l].begin(), c[l].end());
+      af.insert(af.end(), f[l].begin(), f[l].end());
+      if (nb) an.insert(an.end(), (*nb)[l].begin(), (*nb)[l].end());
+    }
+    P.begin[nlev] = (int)ac.size();
+    int e;
+    if ((e = upload_vec(&P.coarse, ac, st)) || (e = upload_vec(&P.fine, af, st)) ||
+        (nb && (e = upload_vec(&P.nb, an, st))))
       return e;
-    ctx->res[l].n = (int)rc_[l].size();
-    ctx->pro[l].n = (int)pc[l].size();
-  }
+    CK(cudaStreamSynchronize(st));  // the copies read the vectors above
+    return IBGPU_OK;
+  };
+  int e;
+  if ((e = pack(ctx->res, rc_, rf, nullptr)) || (e = pack(ctx->pro, pc, pf, &pn))) return e;
   CK(cudaStreamSynchronize(st));
   return IBGPU_OK;
 }

@@ -24,6 +24,42 @@ constexpr int kReg = kTile + 2 * kHalo;  // 20: tile plus a 2-cell halo
 constexpr int kXFaces = kTile * (kTile + 1);
 constexpr int kYFaces = (kTile + 1) * kTile;
 
+// Programmatic dependent launch: a kernel of the step lets the next one be
+// set up as soon as all its CTAs run, and waits for the previous one to have
+// completed before it reads or writes anything that the step changes (mesh
+// tables, which no kernel of a run writes, may be read before).
+__device__ __forceinline__ void dep_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void dep_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+void launch_dep(bool dep, cudaStream_t st, dim3 grid, dim3 block, void (*kernel)(P...),
+                const A &...args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = dep ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// What a step's first stage resets (StageArgs::reset); nothing reads these
+// words before the step's final stage.
+__device__ __forceinline__ void step_reset(const StageArgs &a) {
+  if (a.reset && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (a.reset & 1)
+      for (int c = 0; c < 5; ++c) a.diag->res_bits[c] = 0ull;
+    if (a.reset & 2) a.diag->cfl_bits = (unsigned long long)__double_as_longlong(10000.0);
+  }
+}
+
 __device__ __forceinline__ void raise_error(DevDiag *d, int phase, int check, int slot) {
   unsigned long long key = ((unsigned long long)phase << 40) |
                            ((unsigned long long)check << 32) | (unsigned)slot;
@@ -169,6 +205,9 @@ __global__ void __launch_bounds__(kTileCells) stage_kernel(StageArgs a, CaseCons
   const int tile = a.tile_begin + blockIdx.x;
   const int lvl = a.tile_level[tile];
   const LevelConst &L = cc.lev[lvl];
+  dep_begin();
+  dep_wait();
+  step_reset(a);
 
   // ---- stage the stencil region (tile + 2-cell halo, corners not needed)
   for (int r = tid; r < kReg * kReg; r += kTileCells) {
@@ -520,8 +559,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
     Q4<R> h = {R(0), R(0), R(0), R(0)};
     if (UNI) {
       // every load before the first store
-      if (own) c = Q4<R>{(R)__ldg(in0 + os), (R)__ldg(in1 + os), (R)__ldg(in2 + os), (R)__ldg(in3 + os)};
-      if (side < 4) h = Q4<R>{(R)__ldg(in0 + hs), (R)__ldg(in1 + hs), (R)__ldg(in2 + hs), (R)__ldg(in3 + hs)};
+      if (own) c = Q4<R>{(R)in0[os], (R)in1[os], (R)in2[os], (R)in3[os]};
+      if (side < 4) h = Q4<R>{(R)in0[hs], (R)in1[hs], (R)in2[hs], (R)in3[hs]};
     } else {
       // presence flags first, then the state of the present cells: the
       // stage input where the stages write it, else the step state
@@ -749,6 +788,7 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
                                   (side == 0 ? 1 : side == 1 ? 7 : side == 2 ? 3 : 5))
                           : -1;
 
+  dep_wait();
   {
     // U^n of the tile's own cells, which the update phase reads after the
     // faces, into L1 now (FP64 step 0.798 -> 0.779 ms)
@@ -767,6 +807,7 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
                                                     (tid % kLines) * (128 / (int)sizeof(TI))));
   }
 
+  step_reset(a);
   if (uni) stage_tile<R, LIM, VISC, FINAL, TI, NT, true>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
   else stage_tile<R, LIM, VISC, FINAL, TI, NT, false>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
 }
@@ -776,6 +817,7 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
 template <typename R, int LIM, bool VISC, bool FINAL, typename TI>
 __global__ void __launch_bounds__(StageThreads<R>::value, stage_min_blocks<R, StageThreads<R>::value>())
     stage_kernel_fast(StageArgs a, CaseConst cc) {
+  dep_begin();
   stage_tile_fast<R, LIM, VISC, FINAL, TI>(a, a.v, cc, a.tile_begin + blockIdx.x, a.phase,
                                            a.v.cfl_next, a.prefetch);
 }
@@ -811,6 +853,8 @@ __global__ void __launch_bounds__(NT, stage_min_blocks<R, NT>())
                        const int *__restrict__ phase_base, int table) {
   // phase_base[0]: 8 x the step index; phase_base[1]: 1 when this step's
   // final stage folds in the next step's CFL pass of the cases that allow it
+  dep_begin();
+  dep_wait();
   const int pb = phase_base[0], fold_step = phase_base[1];
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const int2 it = work[w];
@@ -838,6 +882,8 @@ __global__ void __launch_bounds__(NT, stage_min_blocks<R, NT>())
 // (NS_Solver.cpp:196-280): a per-cell bound, a warp-shuffle and block min and
 // one atomic per block (positive doubles order like their bit patterns).
 __global__ void __launch_bounds__(256) cfl_kernel(CflArgs a, CaseConst cc) {
+  dep_begin();
+  dep_wait();
   double best = 10000.0;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < a.nslots;
        s += (int64_t)gridDim.x * blockDim.x) {
@@ -854,28 +900,26 @@ __global__ void __launch_bounds__(256) cfl_kernel(CflArgs a, CaseConst cc) {
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = sred[w] < b ? sred[w] : b;
-    atomicMin(&a.diag->cfl_bits, b);
+    atomicMin(&a.diag->cfl_next_bits, b);
   }
 }
 
 // Per-step reset of the step's reductions (the dt and any earlier abort
-// carry over between the steps of one run).
+// carry over between the steps of one run); for steps whose first stage does
+// not do it.
 __global__ void step_begin_kernel(DevDiag *d) {
+  dep_begin();
+  dep_wait();
   d->cfl_bits = (unsigned long long)__double_as_longlong(10000.0);
   for (int c = 0; c < 5; ++c) d->res_bits[c] = 0ull;
 }
 
-// dt = min(CFL_dt, dt*dt_ratio) (NS_Solver.cpp:263)
-__global__ void finalize_dt_kernel(DevDiag *d, CaseConst cc) {
-  double cdt = __longlong_as_double((long long)d->cfl_bits);
-  double cand = d->dt * cc.dt_ratio;
-  d->dt = (cand < cdt) ? cand : cdt;
-}
-
-// The CFL pass of a step whose bound the previous step's final stage
-// accumulated (cfl_next_bits): take it, reset the accumulator for this
-// step's final stage, and finalise dt.
+// dt = min(CFL_dt, dt*dt_ratio) (NS_Solver.cpp:263) from the bound that the
+// CFL pass or the previous step's final stage accumulated, whose accumulator
+// starts over.
 __global__ void take_folded_cfl_kernel(DevDiag *d, CaseConst cc) {
+  dep_begin();
+  dep_wait();
   d->cfl_bits = d->cfl_next_bits;
   d->cfl_next_bits = (unsigned long long)__double_as_longlong(10000.0);
   double cdt = __longlong_as_double((long long)d->cfl_bits);
@@ -967,57 +1011,57 @@ __global__ void gather_state4_kernel(double *rows, const int32_t *cell_slot, int
 #ifdef IBGPU_FAST_BUILD
 template <typename R, int LIM, typename TI>
 static void launch_stage_ti(const StageArgs &a, const CaseConst &cc, int ntiles, bool visc,
-                            bool final_stage, cudaStream_t st) {
+                            bool final_stage, cudaStream_t st, bool dep) {
   dim3 grid(ntiles), block(StageThreads<R>::value);
   if (visc) {
-    if (final_stage) stage_kernel_fast<R, LIM, true, true, TI><<<grid, block, 0, st>>>(a, cc);
-    else stage_kernel_fast<R, LIM, true, false, TI><<<grid, block, 0, st>>>(a, cc);
+    if (final_stage) launch_dep(dep, st, grid, block, stage_kernel_fast<R, LIM, true, true, TI>, a, cc);
+    else launch_dep(dep, st, grid, block, stage_kernel_fast<R, LIM, true, false, TI>, a, cc);
   } else {
-    if (final_stage) stage_kernel_fast<R, LIM, false, true, TI><<<grid, block, 0, st>>>(a, cc);
-    else stage_kernel_fast<R, LIM, false, false, TI><<<grid, block, 0, st>>>(a, cc);
+    if (final_stage) launch_dep(dep, st, grid, block, stage_kernel_fast<R, LIM, false, true, TI>, a, cc);
+    else launch_dep(dep, st, grid, block, stage_kernel_fast<R, LIM, false, false, TI>, a, cc);
   }
 }
 
 // in32: the stage input is the mixed build's FP32 stage buffer
 template <typename R, int LIM>
 static void launch_stage_t(const StageArgs &a, const CaseConst &cc, int ntiles, bool visc,
-                           bool final_stage, bool in32, cudaStream_t st) {
+                           bool final_stage, bool in32, cudaStream_t st, bool dep) {
   if constexpr (sizeof(R) == 4) {
     if (in32) {
-      launch_stage_ti<R, LIM, float>(a, cc, ntiles, visc, final_stage, st);
+      launch_stage_ti<R, LIM, float>(a, cc, ntiles, visc, final_stage, st, dep);
       return;
     }
   }
-  launch_stage_ti<R, LIM, double>(a, cc, ntiles, visc, final_stage, st);
+  launch_stage_ti<R, LIM, double>(a, cc, ntiles, visc, final_stage, st, dep);
 }
 #else
 template <typename R, int LIM>
 static void launch_stage_t(const StageArgs &a, const CaseConst &cc, int ntiles, bool visc,
-                           bool final_stage, bool, cudaStream_t st) {
+                           bool final_stage, bool, cudaStream_t st, bool dep) {
   dim3 grid(ntiles), block(kTileCells);
   if (visc) {
-    if (final_stage) stage_kernel<R, LIM, true, true><<<grid, block, 0, st>>>(a, cc);
-    else stage_kernel<R, LIM, true, false><<<grid, block, 0, st>>>(a, cc);
+    if (final_stage) launch_dep(dep, st, grid, block, stage_kernel<R, LIM, true, true>, a, cc);
+    else launch_dep(dep, st, grid, block, stage_kernel<R, LIM, true, false>, a, cc);
   } else {
-    if (final_stage) stage_kernel<R, LIM, false, true><<<grid, block, 0, st>>>(a, cc);
-    else stage_kernel<R, LIM, false, false><<<grid, block, 0, st>>>(a, cc);
+    if (final_stage) launch_dep(dep, st, grid, block, stage_kernel<R, LIM, false, true>, a, cc);
+    else launch_dep(dep, st, grid, block, stage_kernel<R, LIM, false, false>, a, cc);
   }
 }
 #endif
 
 void launch_stage(const StageArgs &a, const CaseConst &cc, int ntiles, int limiter, bool visc,
-                  bool final_stage, bool mixed, int stage, cudaStream_t st) {
+                  bool final_stage, bool mixed, int stage, cudaStream_t st, bool dep) {
   if (ntiles <= 0) return;
 #ifndef IBGPU_FAST_BUILD
   mixed = false;  // the exact build is FP64 only
 #endif
   const bool in32 = mixed && stage > 0;
   if (mixed) {
-    if (limiter == LIM_MINMOD) launch_stage_t<float, LIM_MINMOD>(a, cc, ntiles, visc, final_stage, in32, st);
-    else launch_stage_t<float, LIM_VANLEER>(a, cc, ntiles, visc, final_stage, in32, st);
+    if (limiter == LIM_MINMOD) launch_stage_t<float, LIM_MINMOD>(a, cc, ntiles, visc, final_stage, in32, st, dep);
+    else launch_stage_t<float, LIM_VANLEER>(a, cc, ntiles, visc, final_stage, in32, st, dep);
   } else {
-    if (limiter == LIM_MINMOD) launch_stage_t<double, LIM_MINMOD>(a, cc, ntiles, visc, final_stage, false, st);
-    else launch_stage_t<double, LIM_VANLEER>(a, cc, ntiles, visc, final_stage, false, st);
+    if (limiter == LIM_MINMOD) launch_stage_t<double, LIM_MINMOD>(a, cc, ntiles, visc, final_stage, false, st, dep);
+    else launch_stage_t<double, LIM_VANLEER>(a, cc, ntiles, visc, final_stage, false, st, dep);
   }
 }
 
@@ -1246,19 +1290,21 @@ void launch_set_phase_base(int *phase_base, int value, int fold, cudaStream_t st
 }
 #endif
 
-void launch_cfl(const CflArgs &a, const CaseConst &cc, int nsm, cudaStream_t st) {
+void launch_cfl(const CflArgs &a, const CaseConst &cc, int nsm, cudaStream_t st, bool dep) {
   int64_t blocks = (a.nslots + 255) / 256;
   int64_t cap = (int64_t)nsm * 8;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  cfl_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, cc);
-  finalize_dt_kernel<<<1, 1, 0, st>>>(a.diag, cc);
+  launch_dep(dep, st, (unsigned)blocks, 256, cfl_kernel, a, cc);
+  launch_dep(true, st, 1, 1, take_folded_cfl_kernel, a.diag, cc);
 }
 
-void launch_step_begin(DevDiag *d, cudaStream_t st) { step_begin_kernel<<<1, 1, 0, st>>>(d); }
+void launch_step_begin(DevDiag *d, cudaStream_t st, bool dep) {
+  launch_dep(dep, st, 1, 1, step_begin_kernel, d);
+}
 
-void launch_take_folded_cfl(DevDiag *d, const CaseConst &cc, cudaStream_t st) {
-  take_folded_cfl_kernel<<<1, 1, 0, st>>>(d, cc);
+void launch_take_folded_cfl(DevDiag *d, const CaseConst &cc, cudaStream_t st, bool dep) {
+  launch_dep(dep, st, 1, 1, take_folded_cfl_kernel, d, cc);
 }
 
 void launch_scatter(const double *rows, const int32_t *cell_slot, const uint8_t *alias, int64_t n,

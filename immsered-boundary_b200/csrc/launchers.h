@@ -9,13 +9,18 @@
 
 namespace ibgpu {
 
+// dep: the launch may be set up while the previous kernel of the stream still
+// runs (programmatic dependent launch); every kernel of the step waits for
+// its predecessor on the device before it touches the state, so the order of
+// the work is the stream's either way.  A run's first launch passes false.
 #define IBGPU_DECLARE_LAUNCHERS(NS)                                                           \
   namespace NS {                                                                              \
   void launch_stage(const StageArgs &a, const CaseConst &cc, int ntiles, int limiter,         \
-                    bool visc, bool final_stage, bool mixed, int stage, cudaStream_t st);     \
-  void launch_cfl(const CflArgs &a, const CaseConst &cc, int nsm, cudaStream_t st);           \
-  void launch_step_begin(DevDiag *d, cudaStream_t st);                                         \
-  void launch_take_folded_cfl(DevDiag *d, const CaseConst &cc, cudaStream_t st);              \
+                    bool visc, bool final_stage, bool mixed, int stage, cudaStream_t st,      \
+                    bool dep);                                                                \
+  void launch_cfl(const CflArgs &a, const CaseConst &cc, int nsm, cudaStream_t st, bool dep); \
+  void launch_step_begin(DevDiag *d, cudaStream_t st, bool dep);                               \
+  void launch_take_folded_cfl(DevDiag *d, const CaseConst &cc, cudaStream_t st, bool dep);    \
   void launch_scatter(const double *rows, const int32_t *cell_slot, const uint8_t *alias,     \
                       int64_t n, double *const s0[kStateFields], int nsm, cudaStream_t st);   \
   void launch_gather(double *rows, const int32_t *cell_slot, int64_t n,                       \
@@ -25,13 +30,13 @@ namespace ibgpu {
                        int nsm, cudaStream_t st);                                             \
   void launch_gather4(double *rows, const int32_t *cell_slot, int64_t n,                      \
                       double *const s0[kStateFields], int nsm, cudaStream_t st);              \
-  void launch_restrict(const PairArgs &a, const CaseConst &cc, cudaStream_t st);               \
-  void launch_prolong(const PairArgs &a, const CaseConst &cc, cudaStream_t st);                \
-  void launch_bc(const BcArgs &a, const CaseConst &cc, cudaStream_t st);                       \
-  void launch_ib(const IbArgs &a, const CaseConst &cc, cudaStream_t st);                       \
+  void launch_restrict(const PairArgs &a, const CaseConst &cc, cudaStream_t st, bool dep);     \
+  void launch_prolong(const PairArgs &a, const CaseConst &cc, cudaStream_t st, bool dep);      \
+  void launch_bc(const BcArgs &a, const CaseConst &cc, cudaStream_t st, bool dep);             \
+  void launch_ib(const IbArgs &a, const CaseConst &cc, cudaStream_t st, bool dep);             \
   void launch_forces(const ForceArgs &a, const CaseConst &cc, cudaStream_t st);                \
   void launch_viscous(const ViscArgs &a, const CaseConst &cc, int ntiles, bool mixed,          \
-                      cudaStream_t st);                                                        \
+                      cudaStream_t st, bool dep);                                              \
   }
 
 IBGPU_DECLARE_LAUNCHERS(fast)

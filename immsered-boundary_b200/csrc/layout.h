@@ -71,8 +71,9 @@ struct DevDiag {
   unsigned long long cfl_bits;
   unsigned long long res_bits[5];
   unsigned long long err_key;  // ~0ull: no error
-  // CFL bound of the next step, accumulated by a final stage that computes
-  // it (StageArgs::cfl_next) for single-level runs without bodies
+  // CFL bound being accumulated: by the CFL pass, or for the next step by a
+  // final stage that computes it (StageArgs::cfl_next) in single-level runs
+  // without bodies; 10000 outside
   unsigned long long cfl_next_bits;
 };
 
@@ -109,6 +110,9 @@ struct StageArgs {
   // single-case fast stage: warm L2 with the stage input of tile + prefetch,
   // about one wave of resident CTAs ahead (0: off)
   int prefetch;
+  // first stage of a step after a run's first: what it resets for the step
+  // (bit 0 the residual maxima, bit 1 the CFL bound of a step without a pass)
+  int reset;
   // last member: the batched stage's constant-memory table keeps each case's
   // arguments up to here once and its StageVar records per stage
   StageVar v;

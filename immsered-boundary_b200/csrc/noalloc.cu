@@ -71,6 +71,7 @@ __global__ void noalloc_setup_kernel(int ntx, int nty, int32_t *nb, int32_t *lvl
     diag->dt = dt;
     double cfl0 = 10000.0;
     diag->cfl_bits = (unsigned long long)__double_as_longlong(cfl0);
+    diag->cfl_next_bits = diag->cfl_bits;
     for (int c = 0; c < 5; ++c) diag->res_bits[c] = 0ull;
     diag->err_key = ~0ull;
   }
@@ -190,8 +191,8 @@ extern "C" int ibgpu_step_periodic_noalloc(const ibgpu_case *cs, int ts, int nx,
     ca.nslots = nslots;
     ca.phase = 1;
     ca.diag = d_diag;
-    if (exact) exact::launch_cfl(ca, cc, nsm, st);
-    else fast::launch_cfl(ca, cc, nsm, st);
+    if (exact) exact::launch_cfl(ca, cc, nsm, st, true);
+    else fast::launch_cfl(ca, cc, nsm, st, true);
   }
   StageArgs sa;
   std::memset(&sa, 0, sizeof(sa));
@@ -214,8 +215,8 @@ extern "C" int ibgpu_step_periodic_noalloc(const ibgpu_case *cs, int ts, int nx,
     }
     sa.v.tp = cs->tp[k];
     sa.phase = 2 + k;
-    if (exact) exact::launch_stage(sa, cc, ntiles, cs->limiter, false, fin, false, k, st);
-    else fast::launch_stage(sa, cc, ntiles, cs->limiter, false, fin, mixed, k, st);
+    if (exact) exact::launch_stage(sa, cc, ntiles, cs->limiter, false, fin, false, k, st, true);
+    else fast::launch_stage(sa, cc, ntiles, cs->limiter, false, fin, mixed, k, st, true);
   }
   noalloc_rows_out_kernel<<<(nx * ny + 255) / 256, 256, 0, st>>>(d_s0, nx, ny, d_rows_out);
   NA_CK(cudaGetLastError());
