@@ -15,10 +15,7 @@ namespace IBGPU_KNS {
 // AMR::InterfaceRestriction -> PairRestriction_2d -> AverageCell_2d
 // (AMRInterface.cpp:78-110, TwoLevelOp.H:67-87, 225-231): density-weighted
 // mean of the four sons written to the coarse ghost.
-__global__ void restrict_kernel(PairArgs a, CaseConst cc) {
-  dep_begin();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+__device__ __forceinline__ void restrict_pair(const PairArgs &a, const CaseConst &cc, int i) {
   double *const *q = a.s0;
   double roe = 0.0, u = 0.0, v = 0.0, e = 0.0;
   const int4 fine = reinterpret_cast<const int4 *>(a.fine)[i];
@@ -52,10 +49,7 @@ __global__ void restrict_kernel(PairArgs a, CaseConst cc) {
 // 16-22, 35-43): conserved variables of the coarse cell and its x/y
 // neighbours, central gradients (q+ - q-)/2, sons at offsets -/+ 1/4,
 // primitive recovery of each son.
-__global__ void prolong_kernel(PairArgs a, CaseConst cc) {
-  dep_begin();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
+__device__ __forceinline__ void prolong_pair(const PairArgs &a, const CaseConst &cc, int i) {
   double *const *q = a.s0;
   // neighbour order: -x, +x, -y, +y
   double U[5][4];
@@ -104,10 +98,7 @@ __global__ void prolong_kernel(PairArgs a, CaseConst cc) {
 }
 
 // ---- domain boundary ghosts (BCValues::BCBoxTreat, BCValues.H:51-298) ----
-__global__ void bc_kernel(BcArgs a, CaseConst cc) {
-  dep_begin();
-  int i = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.end) return;
+__device__ __forceinline__ void bc_ghost(const BcArgs &a, const CaseConst &cc, int i) {
   double *const *q = a.s0;
   const int g = a.ghost[i], r = a.ref[i];
   const int type = a.type[i];
@@ -173,6 +164,22 @@ __global__ void bc_kernel(BcArgs a, CaseConst cc) {
   q[F_P][g] = p;
   q[F_E][g] = e;
   q[F_T][g] = T;
+}
+
+__global__ void restrict_kernel(PairArgs a, CaseConst cc) {
+  dep_begin();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n) restrict_pair(a, cc, i);
+}
+__global__ void prolong_kernel(PairArgs a, CaseConst cc) {
+  dep_begin();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n) prolong_pair(a, cc, i);
+}
+__global__ void bc_kernel(BcArgs a, CaseConst cc) {
+  dep_begin();
+  const int i = a.begin + blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.end) bc_ghost(a, cc, i);
 }
 
 // ---- immersed-boundary ghost cells (Body::IBConditions_Image) -----------
@@ -359,17 +366,15 @@ __global__ void __launch_bounds__(256) force_sum_kernel(ForceArgs a, CaseConst c
 // One tile per CTA: u, v, T of the tile and a one-cell halo (corners
 // included), every x- and y-face viscous flux into shared memory, then each
 // leaf cell's frozen residual parts vs(high) - vs(low) per direction.
-template <typename R>
-__global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseConst cc) {
+template <typename R, typename A>
+__device__ __forceinline__ void viscous_tile(const A &a, const CaseConst &cc, int tile) {
   constexpr int H = 1, G = kTile + 2 * H;  // 18
   __shared__ R su[G * G], sv[G * G], sT[G * G];
   __shared__ uint8_t sfl[G * G];
   __shared__ R vx[3][kXFaces];  // x-mom, y-mom, energy of x-faces
   __shared__ R vy[3][kYFaces];
   const int tid = threadIdx.x;
-  const int tile = a.tile_begin + blockIdx.x;
   const LevelConst &L = cc.lev[a.tile_level[tile]];
-  dep_begin();
   dep_wait();
   for (int r = tid; r < G * G; r += kTileCells) {
     int rx = r % G - H, ry = r / G - H;
@@ -465,15 +470,96 @@ __global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseCon
   if (sfl[(ly + H) * G + (lx + H)] & CF_NORMAL) {
     const int xlo = ly * (kTile + 1) + lx, xhi = xlo + 1;
     const int ylo = ly * kTile + lx, yhi = ylo + kTile;
-    a.vsd[0 * a.nslots + slot] = 0.0 - 0.0;
-    a.vsd[4 * a.nslots + slot] = 0.0 - 0.0;
+    double *vsd = const_cast<double *>(a.vsd);  // a stage's arguments only read it
+    vsd[0 * a.nslots + slot] = 0.0 - 0.0;
+    vsd[4 * a.nslots + slot] = 0.0 - 0.0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      a.vsd[(int64_t)(1 + c) * a.nslots + slot] = (double)vx[c][xhi] - (double)vx[c][xlo];
-      a.vsd[(int64_t)(5 + c) * a.nslots + slot] = (double)vy[c][yhi] - (double)vy[c][ylo];
+      vsd[(int64_t)(1 + c) * a.nslots + slot] = (double)vx[c][xhi] - (double)vx[c][xlo];
+      vsd[(int64_t)(5 + c) * a.nslots + slot] = (double)vy[c][yhi] - (double)vy[c][ylo];
     }
   }
 }
+
+template <typename R>
+__global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseConst cc) {
+  dep_begin();
+  viscous_tile<R>(a, cc, a.tile_begin + (int)blockIdx.x);
+}
+
+#ifdef IBGPU_FAST_BUILD
+// ---- the same over several cases: each block takes one block of one case
+__global__ void restrict_kernel_batch(const BatchPairs *__restrict__ segs,
+                                      const CaseConst *__restrict__ ccs,
+                                      const int2 *__restrict__ blocks) {
+  dep_begin();
+  const int2 b = blocks[blockIdx.x];
+  const BatchPairs &s = segs[b.x];
+  const int i = b.y + threadIdx.x;
+  if (i < s.a.n) restrict_pair(s.a, ccs[s.c], i);
+}
+__global__ void prolong_kernel_batch(const BatchPairs *__restrict__ segs,
+                                     const CaseConst *__restrict__ ccs,
+                                     const int2 *__restrict__ blocks) {
+  dep_begin();
+  const int2 b = blocks[blockIdx.x];
+  const BatchPairs &s = segs[b.x];
+  const int i = b.y + threadIdx.x;
+  if (i < s.a.n) prolong_pair(s.a, ccs[s.c], i);
+}
+__global__ void bc_kernel_batch(const BatchBc *__restrict__ segs,
+                                const CaseConst *__restrict__ ccs,
+                                const int2 *__restrict__ blocks) {
+  dep_begin();
+  const int2 b = blocks[blockIdx.x];
+  const BatchBc &s = segs[b.x];
+  const int i = b.y + threadIdx.x;
+  if (i < s.a.end) bc_ghost(s.a, ccs[s.c], i);
+}
+// one CTA per case (each of at most kIbBlock cells)
+__global__ void __launch_bounds__(kIbBlock)
+    ib_kernel_batch(const BatchIb *__restrict__ segs, const CaseConst *__restrict__ ccs) {
+  dep_begin();
+  dep_wait();
+  const BatchIb &s = segs[blockIdx.x];
+  const int i = threadIdx.x;
+  double o[6];
+  if (i < s.a.n) ib_cell(s.a, ccs[s.c], i, o);
+  __syncthreads();
+  if (i < s.a.n) ib_put(s.a, i, o);
+}
+template <typename R>
+__global__ void __launch_bounds__(kTileCells)
+    viscous_kernel_batch(const StageArgs *__restrict__ args, const CaseConst *__restrict__ ccs,
+                         const int2 *__restrict__ work, int nstages) {
+  dep_begin();
+  const int2 it = work[blockIdx.x];
+  viscous_tile<R>(args[it.x * nstages], ccs[it.x], it.y);
+}
+
+void launch_pairs_batch(const BatchPairs *segs, const CaseConst *ccs, const int2 *blocks,
+                        int nblocks, bool prolong, cudaStream_t st) {
+  if (nblocks <= 0) return;
+  launch_dep(true, st, nblocks, kBatchBlock, prolong ? prolong_kernel_batch : restrict_kernel_batch,
+             segs, ccs, blocks);
+}
+void launch_bc_batch(const BatchBc *segs, const CaseConst *ccs, const int2 *blocks, int nblocks,
+                     cudaStream_t st) {
+  if (nblocks > 0) launch_dep(true, st, nblocks, kBatchBlock, bc_kernel_batch, segs, ccs, blocks);
+}
+bool launch_ib_batch(const BatchIb *segs, const CaseConst *ccs, int ncases, int most,
+                     cudaStream_t st) {
+  if (most > kIbBlock) return false;
+  if (ncases > 0) launch_dep(true, st, ncases, (most + 31) / 32 * 32, ib_kernel_batch, segs, ccs);
+  return true;
+}
+void launch_viscous_batch(const StageArgs *args, const CaseConst *ccs, const int2 *work, int nwork,
+                          int nstages, bool mixed, cudaStream_t st) {
+  if (nwork <= 0) return;
+  if (mixed) launch_dep(true, st, nwork, kTileCells, viscous_kernel_batch<float>, args, ccs, work, nstages);
+  else launch_dep(true, st, nwork, kTileCells, viscous_kernel_batch<double>, args, ccs, work, nstages);
+}
+#endif
 
 // ---- launchers ---------------------------------------------------------------
 void launch_restrict(const PairArgs &a, const CaseConst &cc, cudaStream_t st, bool dep) {

@@ -3,6 +3,7 @@
 // reference main loop and NS_Solver::TimeMarching (main.cpp:84-116,
 // NS_Solver.H:657-702).
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -1072,6 +1073,50 @@ bool stage_resets(const ibgpu_ctx *ctx, int ts) {
   return any && cs.nstages > 1;
 }
 
+// Arguments of the fills' launches: pairs of levels [l0, l1), one dependency
+// wave of the domain ghosts, the immersed-boundary cells.
+PairArgs pair_args(const ibgpu_ctx *ctx, const ibgpu_ctx::DevPairs &P, bool prolong, int l0,
+                   int l1) {
+  PairArgs pa;
+  pa.coarse = P.coarse + P.begin[l0];
+  pa.fine = P.fine + 4 * (size_t)P.begin[l0];
+  pa.nb = prolong ? P.nb + 4 * (size_t)P.begin[l0] : nullptr;
+  pa.n = P.begin[l1] - P.begin[l0];
+  for (int f = 0; f < kStateFields; ++f) pa.s0[f] = ctx->d_s0[f];
+  return pa;
+}
+BcArgs bc_args(const ibgpu_ctx *ctx, const std::pair<int, int> &wave) {
+  BcArgs ba;
+  ba.ghost = ctx->d_bc_ghost;
+  ba.ref = ctx->d_bc_ref;
+  ba.type = ctx->d_bc_type;
+  ba.face = ctx->d_bc_face;
+  ba.nmv = ctx->d_bc_nmv;
+  ba.facevar = ctx->d_facevar;
+  ba.begin = wave.first;
+  ba.end = wave.second;
+  ba.backpressure = ctx->backpressure;
+  ba.cos_in = ctx->cos_in;
+  ba.sin_in = ctx->sin_in;
+  for (int f = 0; f < kStateFields; ++f) ba.s0[f] = ctx->d_s0[f];
+  return ba;
+}
+// phase: the step's abort-order phase base, 0 when it is read from the
+// batch's device counters (phase_base)
+IbArgs ib_args(const ibgpu_ctx *ctx, int phase, const int *phase_base) {
+  IbArgs ia;
+  ia.cell = ctx->d_ib_cell;
+  ia.intp = ctx->d_ib_intp;
+  ia.cellf = ctx->d_ib_f;
+  ia.out = ctx->d_ib_out;
+  ia.n = ctx->n_ib;
+  for (int f = 0; f < kStateFields; ++f) ia.s0[f] = ctx->d_s0[f];
+  ia.phase = phase;
+  ia.phase_base = phase_base;
+  ia.diag = ctx->d_diag;
+  return ia;
+}
+
 // Everything of step ts before the stages (main.cpp:87-89 and the frozen
 // part of NS_Solver::TimeMarching): restriction and prolongation on their
 // schedules, immersed-body ghosts, CFL dt, domain ghosts and the viscous flux
@@ -1080,8 +1125,7 @@ bool stage_resets(const ibgpu_ctx *ctx, int ts) {
 // most of the chip idle for its launch.  dep: whether the next launch may
 // overlap its predecessor's end (false for the first of a run).
 int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer &tm, bool &dep,
-                     bool batched = false, bool fresh_cfl = false,
-                     const int *phase_base = nullptr) {
+                     bool batched = false, bool fresh_cfl = false) {
   const ibgpu_case &cs = ctx->cs;
   const bool exact = cs.precision == IBGPU_FP64_EXACT;
   const bool mixed = cs.precision == IBGPU_MIXED;
@@ -1105,12 +1149,7 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
         [&](int l) { return ts % every[l + 1] == left[l + 1] && P.count(l) > 0; },
         [&](int l) { return P.joins[l] != 0; },
         [&](int l0, int l1) {
-          PairArgs pa;
-          pa.coarse = P.coarse + P.begin[l0];
-          pa.fine = P.fine + 4 * (size_t)P.begin[l0];
-          pa.nb = pass ? P.nb + 4 * (size_t)P.begin[l0] : nullptr;
-          pa.n = P.begin[l1] - P.begin[l0];
-          for (int f = 0; f < kStateFields; ++f) pa.s0[f] = ctx->d_s0[f];
+          const PairArgs pa = pair_args(ctx, P, pass != 0, l0, l1);
           if (pass) {
             if (exact) exact::launch_prolong(pa, ctx->cc, st, dep);
             else fast::launch_prolong(pa, ctx->cc, st, dep);
@@ -1126,18 +1165,7 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
   }
   // Body::IBConditions_Image (static bodies): IB ghost cells of the finest level
   if (ctx->n_ib > 0) {
-    IbArgs ia;
-    ia.cell = ctx->d_ib_cell;
-    ia.intp = ctx->d_ib_intp;
-    ia.cellf = ctx->d_ib_f;
-    ia.out = ctx->d_ib_out;
-    ia.n = ctx->n_ib;
-    for (int f = 0; f < kStateFields; ++f) ia.s0[f] = ctx->d_s0[f];
-    // the abort-order phase of this step: from the host, or (a captured
-    // batch step replayed for every step) from the batch's device counter
-    ia.phase = phase_base ? 0 : pbase + 0;
-    ia.phase_base = phase_base;
-    ia.diag = ctx->d_diag;
+    const IbArgs ia = ib_args(ctx, pbase, nullptr);
     if (exact) exact::launch_ib(ia, ctx->cc, st, dep);
     else fast::launch_ib(ia, ctx->cc, st, dep);
     dep = true;
@@ -1174,19 +1202,7 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
   for (int l = 0; l < cs.nlevels && l < (int)ctx->bc_waves.size(); ++l) {
     if (ts % cs.march_step[l] != cs.march_left[l]) continue;
     for (auto &w : ctx->bc_waves[l]) {
-      BcArgs ba;
-      ba.ghost = ctx->d_bc_ghost;
-      ba.ref = ctx->d_bc_ref;
-      ba.type = ctx->d_bc_type;
-      ba.face = ctx->d_bc_face;
-      ba.nmv = ctx->d_bc_nmv;
-      ba.facevar = ctx->d_facevar;
-      ba.begin = w.first;
-      ba.end = w.second;
-      ba.backpressure = ctx->backpressure;
-      ba.cos_in = ctx->cos_in;
-      ba.sin_in = ctx->sin_in;
-      for (int f = 0; f < kStateFields; ++f) ba.s0[f] = ctx->d_s0[f];
+      const BcArgs ba = bc_args(ctx, w);
       if (exact) exact::launch_bc(ba, ctx->cc, st, dep);
       else fast::launch_bc(ba, ctx->cc, st, dep);
       dep = true;
@@ -1444,6 +1460,8 @@ int ibgpu_step_result(ibgpu_ctx *ctx, double *dt, ibgpu_diag *diag) {
 // ---------------------------------------------------------------------------
 // Batched cases: the stage launches of every case merged into one persistent
 // launch over a (case, tile) work list, replayed from a CUDA graph.
+constexpr int kMaxBatchPeriod = 4096;  // schedule phases a batch prepares launches for
+
 struct ibgpu_batch {
   std::vector<ibgpu_ctx *> cases;
   cudaStream_t stream = nullptr;
@@ -1454,14 +1472,25 @@ struct ibgpu_batch {
   int *d_phase_base = nullptr;
   std::vector<int2 *> d_work;      // per schedule phase r = ts % period
   std::vector<int> nwork;
-  // whole-step graphs (every case's ghost fills and viscous pass on parallel
-  // branches, then the merged CFL and stage launches), captured on first use
-  // per (ts % full_period, CFL variant)
+  // whole-step graphs (the cases' ghost fills and viscous pass, the CFL pass
+  // and the stages, each launch over all cases), captured on first use per
+  // (ts % full_period, CFL variant)
   std::map<int, cudaGraphExec_t> graphs;
   bool graphs_ready = false;  // every phase's graphs captured (first run after tuning)
   int full_period = 1;  // every schedule of every case repeats with it
-  std::vector<cudaStream_t> fork;  // branches of the captured steps
-  std::vector<cudaEvent_t> ev_fork_join;
+  // the fills of the cases that are due at ts % full_period == q, one launch
+  // after another: blocks of the segments below
+  struct Fill {
+    int kind;  // 0 restriction, 1 prolongation, 2 domain ghosts
+    int2 *blocks;
+    int n;
+  };
+  std::vector<std::vector<Fill>> fills;
+  std::vector<int2 *> fill_blocks;  // owned (several phases share one)
+  BatchPairs *d_pairs = nullptr;
+  BatchBc *d_bcs = nullptr;
+  BatchIb *d_ibs = nullptr;
+  int n_ibs = 0, most_ib = 0;
   int2 *d_cfl_work = nullptr;      // every tile of every case
   int ncfl = 0, dt_var_step = 1;
   // cases with different CFL intervals (each dividing the schedule period):
@@ -1496,10 +1525,15 @@ struct ibgpu_batch {
   }
   void release() {
     drop_graphs();
-    for (auto f : fork) cudaStreamDestroy(f);
-    fork.clear();
-    for (auto e : ev_fork_join) cudaEventDestroy(e);
-    ev_fork_join.clear();
+    for (auto w : fill_blocks) cudaFree(w);
+    fill_blocks.clear();
+    fills.clear();
+    cudaFree(d_pairs);
+    cudaFree(d_bcs);
+    cudaFree(d_ibs);
+    d_pairs = nullptr;
+    d_bcs = nullptr;
+    d_ibs = nullptr;
     for (auto w : d_work) cudaFree(w);
     d_work.clear();
     cudaFree(d_cfl_work);
@@ -1671,14 +1705,126 @@ int write_batch_table(ibgpu_batch *b, const std::vector<StageArgs> &args,
   return IBGPU_OK;
 }
 
-// One graph per schedule phase holding the nstages merged stage launches;
-// without a capturable stream the launches are issued directly.
-// The graph of one whole batch step at schedule phase q = ts % full_period
-// with CFL variant cfl, captured on first use: the cases' ghost fills and
-// viscous passes (their abort phase read from the batch's device counter)
-// forked onto the batch's branch streams, joined, then the merged CFL and
-// stage launches.  Nothing in it depends on the step index except through
-// the device counter, so one capture serves every step of that phase.
+// One batch step at schedule phase q = ts % full_period with CFL variant
+// cfl: the step's index and resets, then each kind of fill, the viscous pass,
+// the CFL pass and the stages, every launch over all the cases it is due for
+// (a launch per case and level left most of the chip idle: 64 us a step of
+// six small airfoils).  Everything that depends on the step's index reads it
+// from the batch's device counters.
+int enqueue_batch_step(ibgpu_batch *b, int q, int cfl, cudaStream_t st) {
+  fast::launch_batch_step(b->d_phase_base, b->d_args, (int)b->cases.size(), b->nstages, st);
+  CK(cudaGetLastError());
+  auto run_fills = [&](bool domain) -> int {
+    for (const auto &f : b->fills[q]) {
+      if ((f.kind == 2) != domain) continue;
+      if (domain) fast::launch_bc_batch(b->d_bcs, b->d_ccs, f.blocks, f.n, st);
+      else fast::launch_pairs_batch(b->d_pairs, b->d_ccs, f.blocks, f.n, f.kind == 1, st);
+      CK(cudaGetLastError());
+    }
+    return IBGPU_OK;
+  };
+  int rc = run_fills(false);
+  if (rc) return rc;
+  if (!fast::launch_ib_batch(b->d_ibs, b->d_ccs, b->n_ibs, b->most_ib, st)) {
+    for (ibgpu_ctx *c : b->cases)
+      if (c->n_ib > 0) fast::launch_ib(ib_args(c, 0, b->d_phase_base), c->cc, st, true);
+  }
+  CK(cudaGetLastError());
+  if ((rc = run_fills(true))) return rc;
+  const int r = q % b->period;
+  if (b->visc) {
+    fast::launch_viscous_batch(b->d_args, b->d_ccs, b->d_work[r], b->nwork[r], b->nstages,
+                               b->mixed, st);
+    CK(cudaGetLastError());
+  }
+  return enqueue_batch_stages(b, r, cfl, st);
+}
+
+// The lists of enqueue_batch_step for every schedule phase: the launches a
+// case's own step makes (levels that run together, dependency waves), the
+// k-th of every case merged into one.
+int build_fills(ibgpu_batch *b) {
+  std::vector<BatchPairs> pairs;
+  std::vector<BatchBc> bcs;
+  std::vector<BatchIb> ibs;
+  std::map<std::vector<int>, int> known;         // (kind, case, l0, l1 | wave) -> segment
+  std::map<std::vector<int>, int2 *> block_list;  // segments -> their blocks
+  const int n = (int)b->cases.size();
+  b->fills.assign(b->full_period, {});
+  for (int i = 0; i < n; ++i) {
+    ibgpu_ctx *c = b->cases[i];
+    if (c->n_ib <= 0) continue;
+    ibs.push_back(BatchIb{ib_args(c, 0, b->d_phase_base), i});
+    b->most_ib = std::max(b->most_ib, c->n_ib);
+  }
+  for (int q = 0; q < b->full_period; ++q) {
+    for (int kind = 0; kind < 3; ++kind) {
+      std::vector<std::vector<std::array<int, 3>>> rounds;  // (segment, first, end)
+      for (int i = 0; i < n; ++i) {
+        ibgpu_ctx *c = b->cases[i];
+        const ibgpu_case &cs = c->cs;
+        size_t k = 0;
+        auto put = [&](int seg, int first, int end) {
+          if (rounds.size() <= k) rounds.resize(k + 1);
+          rounds[k++].push_back({seg, first, end});
+        };
+        if (kind < 2) {
+          const ibgpu_ctx::DevPairs &P = kind ? c->pro : c->res;
+          const int *every = kind ? cs.prolong_step : cs.average_step;
+          const int *left = kind ? cs.prolong_left : cs.average_left;
+          level_runs(
+              cs.nlevels - 1,
+              [&](int l) { return q % every[l + 1] == left[l + 1] && P.count(l) > 0; },
+              [&](int l) { return P.joins[l] != 0; },
+              [&](int l0, int l1) {
+                auto it = known.emplace(std::vector<int>{kind, i, l0, l1}, (int)pairs.size());
+                if (it.second) pairs.push_back(BatchPairs{pair_args(c, P, kind == 1, l0, l1), i});
+                put(it.first->second, 0, P.begin[l1] - P.begin[l0]);
+                return 0;
+              });
+        } else {
+          for (int l = 0; l < cs.nlevels && l < (int)c->bc_waves.size(); ++l) {
+            if (q % cs.march_step[l] != cs.march_left[l]) continue;
+            for (const auto &w : c->bc_waves[l]) {
+              auto it = known.emplace(std::vector<int>{kind, i, w.first, w.second}, (int)bcs.size());
+              if (it.second) bcs.push_back(BatchBc{bc_args(c, w), i});
+              put(it.first->second, w.first, w.second);
+            }
+          }
+        }
+      }
+      for (const auto &round : rounds) {
+        std::vector<int> key{kind};
+        std::vector<int2> blocks;
+        for (const auto &s : round) {
+          key.push_back(s[0]);
+          for (int f = s[1]; f < s[2]; f += kBatchBlock) blocks.push_back(make_int2(s[0], f));
+        }
+        int2 *&d = block_list[key];
+        if (!d) {
+          int rc = dev_alloc(&d, blocks.size());
+          if (rc) return rc;
+          b->fill_blocks.push_back(d);
+          CK(cudaMemcpy(d, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice));
+        }
+        b->fills[q].push_back({kind, d, (int)blocks.size()});
+      }
+    }
+  }
+  b->n_ibs = (int)ibs.size();
+  int rc;
+  if ((rc = dev_alloc(&b->d_pairs, pairs.size())) || (rc = dev_alloc(&b->d_bcs, bcs.size())) ||
+      (rc = dev_alloc(&b->d_ibs, ibs.size())))
+    return rc;
+  CK(cudaMemcpy(b->d_pairs, pairs.data(), pairs.size() * sizeof(BatchPairs), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(b->d_bcs, bcs.data(), bcs.size() * sizeof(BatchBc), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(b->d_ibs, ibs.data(), ibs.size() * sizeof(BatchIb), cudaMemcpyHostToDevice));
+  return IBGPU_OK;
+}
+
+// The graph of one whole batch step, captured on first use: nothing in it
+// depends on the step's index except through the device counters, so one
+// capture serves every step of that phase.
 int batch_step_graph(ibgpu_batch *b, int q, int cfl, cudaGraphExec_t *out) {
   const int key = q * 3 + cfl;
   auto it = b->graphs.find(key);
@@ -1687,32 +1833,17 @@ int batch_step_graph(ibgpu_batch *b, int q, int cfl, cudaGraphExec_t *out) {
     return IBGPU_OK;
   }
   cudaStream_t st = b->stream;
-  const int nf = (int)b->fork.size();
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  int rc = IBGPU_OK;
-  cudaError_t e = cudaEventRecord(b->ev_fork_join[nf], st);
-  for (int k = 0; k < nf && e == cudaSuccess; ++k) e = cudaStreamWaitEvent(b->fork[k], b->ev_fork_join[nf], 0);
-  for (size_t i = 0; i < b->cases.size() && e == cudaSuccess && !rc; ++i) {
-    RunTimer tm{b->cases[i], b->fork[i % nf], {}, {}};
-    tm.off = true;
-    bool dep = false;
-    rc = enqueue_prestage(b->cases[i], q, 1, b->fork[i % nf], tm, dep, true, false, b->d_phase_base);
-  }
-  for (int k = 0; k < nf && e == cudaSuccess && !rc; ++k) {
-    e = cudaEventRecord(b->ev_fork_join[k], b->fork[k]);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, b->ev_fork_join[k], 0);
-  }
-  if (e == cudaSuccess && !rc) rc = enqueue_batch_stages(b, q % b->period, cfl, st);
-  cudaError_t e2 = cudaStreamEndCapture(st, &g);
+  const int rc = enqueue_batch_step(b, q, cfl, st);
+  const cudaError_t e2 = cudaStreamEndCapture(st, &g);
   if (rc) {
     if (g) cudaGraphDestroy(g);
     return rc;
   }
-  if (e != cudaSuccess) return cuda_fail(e, "batch step capture");
   if (e2 != cudaSuccess) return cuda_fail(e2, "cudaStreamEndCapture");
   cudaGraphExec_t x = nullptr;
-  e = cudaGraphInstantiate(&x, g, 0);
+  const cudaError_t e = cudaGraphInstantiate(&x, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
   b->graphs[key] = x;
@@ -1792,7 +1923,7 @@ int ibgpu_batch_create(ibgpu_ctx *const *cases, int ncases, ibgpu_batch **out) {
         fp = lcm(fp, c->cs.march_step[l]);
         if (l >= 1) fp = lcm(lcm(fp, c->cs.average_step[l]), c->cs.prolong_step[l]);
       }
-      if (fp > 4096) break;
+      if (fp > kMaxBatchPeriod) break;
     }
     b->full_period = fp;
   }
@@ -1824,11 +1955,11 @@ int ibgpu_batch_create(ibgpu_ctx *const *cases, int ncases, ibgpu_batch **out) {
   };
   int rc;
   if ((rc = dev_alloc(&b->d_args, args.size())) || (rc = dev_alloc(&b->d_ccs, ccs.size())) ||
-      (rc = dev_alloc(&b->d_phase_base, 2)))
+      (rc = dev_alloc(&b->d_phase_base, 5)))
     return fail(rc);
   cudaError_t e = cudaMemcpy(b->d_args, args.data(), args.size() * sizeof(StageArgs), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(b->d_ccs, ccs.data(), ccs.size() * sizeof(CaseConst), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(b->d_phase_base, 0, 2 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(b->d_phase_base, 0, 5 * sizeof(int));
   if (e != cudaSuccess) return fail(cuda_fail(e, "batch upload"));
   if ((rc = write_batch_table(b, args, ccs))) return fail(rc);
   // work lists: case-interleaved so the persistent CTAs mix the cases
@@ -1900,18 +2031,7 @@ int ibgpu_batch_create(ibgpu_ctx *const *cases, int ncases, ibgpu_batch **out) {
       if (e != cudaSuccess) return fail(cuda_fail(e, "batch CFL work list"));
     }
   }
-  // branch streams of the captured steps: up to eight, cases round robin
-  {
-    const int nf = std::min(8, ncases);
-    b->fork.assign(nf, nullptr);
-    b->ev_fork_join.assign(nf + 1, nullptr);
-    for (int k = 0; k < nf; ++k)
-      if ((e = cudaStreamCreateWithFlags(&b->fork[k], cudaStreamNonBlocking)) != cudaSuccess)
-        return fail(cuda_fail(e, "batch branch stream"));
-    for (auto &ev : b->ev_fork_join)
-      if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
-        return fail(cuda_fail(e, "batch branch event"));
-  }
+  if (b->full_period <= kMaxBatchPeriod && (rc = build_fills(b))) return fail(rc);
   *out = b;
   return IBGPU_OK;
 }
@@ -1925,11 +2045,12 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
     if ((rc = autotune(b))) return rc;
     b->drop_graphs();  // captured with the previous launch shape
   }
-  // captured whole steps, unless something asks for per-launch timing or the
-  // batch runs on the legacy stream (not capturable); captured before this
-  // run's first work is enqueued
-  bool use_graphs = b->stream != nullptr && !b->timing && b->full_period <= 4096;
-  for (int i = 0; i < n; ++i) use_graphs = use_graphs && !b->cases[i]->timing;
+  // merged launches, captured where the stream can be (the legacy one
+  // cannot); a case with kernel timing enabled, and schedules that repeat too
+  // rarely, take each case's own launches
+  bool merged = b->full_period <= kMaxBatchPeriod;
+  for (int i = 0; i < n; ++i) merged = merged && !b->cases[i]->timing;
+  const bool use_graphs = merged && b->stream != nullptr && !b->timing;
   if (use_graphs && (rc = batch_prepare_graphs(b))) return rc;
   for (int i = 0; i < n; ++i) {
     if (b->cases[i]->download_pending) {
@@ -1944,21 +2065,24 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> sev;
   std::vector<int64_t> marched(n, 0);
+  const int counters[5] = {0, 0, -1, nsteps, b->folds};
+  CK(cudaMemcpyAsync(b->d_phase_base, counters, sizeof(counters), cudaMemcpyHostToDevice, st));
   for (int step = 0; step < nsteps; ++step) {
     const int ts = ts0 + step;
     const int r = ts % b->period;
-    if (step > 0) fast::launch_step_begin_batch(b->d_args, n, b->nstages, st);
     for (int i = 0; i < n; ++i) marched[i] = marched_cells(b->cases[i], ts);
     const bool cfl_now = b->mixed_cfl ? b->ncfl_cases_r[r] > 0 : (ts % b->dt_var_step) == 0;
     const int cfl = !cfl_now ? 0 : (b->folds && step > 0 ? 2 : 1);
-    fast::launch_set_phase_base(b->d_phase_base, 8 * step, b->folds && step + 1 < nsteps, st);
     if (use_graphs) {
       // the whole step as one graph (the stage launches' own timing is not
       // separable then: b->timing runs without graphs)
       cudaGraphExec_t gx = nullptr;
       if ((rc = batch_step_graph(b, ts % b->full_period, cfl, &gx))) return rc;
       CK(cudaGraphLaunch(gx, st));
+    } else if (merged && !b->timing) {
+      if ((rc = enqueue_batch_step(b, ts % b->full_period, cfl, st))) return rc;
     } else {
+      fast::launch_batch_step(b->d_phase_base, b->d_args, n, b->nstages, st);
       for (int i = 0; i < n; ++i) {
         bool dep = false;
         if ((rc = enqueue_prestage(b->cases[i], ts, step, st, tms[i], dep, true))) return rc;

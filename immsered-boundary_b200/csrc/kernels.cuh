@@ -1073,14 +1073,14 @@ static void launch_batch_n(const StageArgs *args, const CaseConst *ccs, const in
   dim3 g(grid), block(NT);
   if (visc) {
     if (final_stage)
-      stage_kernel_batch<R, LIM, true, true, LOOP, TABLE, TI, NT><<<g, block, 0, st>>>(args, ccs, work, nwork, stage, nstages, phase_base, table);
+      launch_dep(true, st, g, block, stage_kernel_batch<R, LIM, true, true, LOOP, TABLE, TI, NT>, args, ccs, work, nwork, stage, nstages, phase_base, table);
     else
-      stage_kernel_batch<R, LIM, true, false, LOOP, TABLE, TI, NT><<<g, block, 0, st>>>(args, ccs, work, nwork, stage, nstages, phase_base, table);
+      launch_dep(true, st, g, block, stage_kernel_batch<R, LIM, true, false, LOOP, TABLE, TI, NT>, args, ccs, work, nwork, stage, nstages, phase_base, table);
   } else {
     if (final_stage)
-      stage_kernel_batch<R, LIM, false, true, LOOP, TABLE, TI, NT><<<g, block, 0, st>>>(args, ccs, work, nwork, stage, nstages, phase_base, table);
+      launch_dep(true, st, g, block, stage_kernel_batch<R, LIM, false, true, LOOP, TABLE, TI, NT>, args, ccs, work, nwork, stage, nstages, phase_base, table);
     else
-      stage_kernel_batch<R, LIM, false, false, LOOP, TABLE, TI, NT><<<g, block, 0, st>>>(args, ccs, work, nwork, stage, nstages, phase_base, table);
+      launch_dep(true, st, g, block, stage_kernel_batch<R, LIM, false, false, LOOP, TABLE, TI, NT>, args, ccs, work, nwork, stage, nstages, phase_base, table);
   }
 }
 
@@ -1186,6 +1186,8 @@ __global__ void __launch_bounds__(kTileCells)
                      const int2 *__restrict__ work, int nwork, int nstages,
                      const int *__restrict__ phase_base) {
   __shared__ unsigned long long sred[kTileCells / 32];
+  dep_begin();
+  dep_wait();
   const int pb = *phase_base;
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const int2 it = work[w];
@@ -1213,6 +1215,8 @@ __global__ void __launch_bounds__(kTileCells)
 // dt = min(CFL_dt, dt*dt_ratio) of every batched case (one thread each)
 __global__ void finalize_dt_batch(const StageArgs *__restrict__ args,
                                   const CaseConst *__restrict__ ccs, int ncases, int nstages) {
+  dep_begin();
+  dep_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncases) return;
   DevDiag *d = args[c * nstages].diag;
@@ -1224,6 +1228,8 @@ __global__ void finalize_dt_batch(const StageArgs *__restrict__ args,
 // the CFL bound each batched case's previous final stage accumulated
 __global__ void take_folded_batch(const StageArgs *__restrict__ args,
                                   const CaseConst *__restrict__ ccs, int ncases, int nstages) {
+  dep_begin();
+  dep_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncases) return;
   DevDiag *d = args[c * nstages].diag;
@@ -1235,22 +1241,39 @@ __global__ void take_folded_batch(const StageArgs *__restrict__ args,
 }
 void launch_take_folded_batch(const StageArgs *args, const CaseConst *ccs, int ncases, int nstages,
                               cudaStream_t st) {
-  take_folded_batch<<<(ncases + 127) / 128, 128, 0, st>>>(args, ccs, ncases, nstages);
+  launch_dep(true, st, (ncases + 127) / 128, 128, take_folded_batch, args, ccs, ncases, nstages);
 }
 
-// per-step reset of the reductions of every batched case
-__global__ void step_begin_batch(const StageArgs *__restrict__ args, int ncases, int nstages) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncases) return;
-  DevDiag *d = args[c * nstages].diag;
-  d->cfl_bits = (unsigned long long)__double_as_longlong(10000.0);
-  for (int k = 0; k < 5; ++k) d->res_bits[k] = 0ull;
+// First launch of every batched step: the step's index and abort-order phase
+// base (8 x the index), whether its final stage folds in the next step's CFL
+// pass, and, after a run's first step, the reset of every case's reductions.
+// c[0], c[1] are what the stages read; c[2] the last step's index (-1 before
+// the first), c[3] the run's steps, c[4] whether the cases fold.
+__global__ void batch_step_kernel(int *c, const StageArgs *__restrict__ args, int ncases,
+                                  int nstages) {
+  dep_begin();
+  dep_wait();
+  const int step = c[2] + 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    c[2] = step;
+    c[0] = 8 * step;
+    c[1] = c[4] && step + 1 < c[3];
+  }
+  if (step > 0)
+    for (int k = threadIdx.x; k < ncases; k += blockDim.x) {
+      DevDiag *d = args[k * nstages].diag;
+      d->cfl_bits = (unsigned long long)__double_as_longlong(10000.0);
+      for (int j = 0; j < 5; ++j) d->res_bits[j] = 0ull;
+    }
 }
 
 // dt of the listed batched cases only (the cases whose CFL pass ran)
 __global__ void finalize_dt_batch_list(const StageArgs *__restrict__ args,
                                        const CaseConst *__restrict__ ccs,
                                        const int *__restrict__ list, int n, int nstages) {
+  dep_begin();
+  dep_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int c = list[k];
@@ -1265,28 +1288,20 @@ void launch_cfl_batch(const StageArgs *args, const CaseConst *ccs, const int2 *w
                       const int *case_list) {
   if (nwork > 0) {
     if (grid < 1 || grid > nwork) grid = nwork;
-    cfl_kernel_batch<<<grid, kTileCells, 0, st>>>(args, ccs, work, nwork, nstages, phase_base);
+    launch_dep(true, st, grid, kTileCells, cfl_kernel_batch, args, ccs, work, nwork, nstages, phase_base);
   }
   if (case_list) {
     if (ncases > 0)
-      finalize_dt_batch_list<<<(ncases + 127) / 128, 128, 0, st>>>(args, ccs, case_list, ncases,
-                                                                    nstages);
+      launch_dep(true, st, (ncases + 127) / 128, 128, finalize_dt_batch_list, args, ccs, case_list,
+                 ncases, nstages);
   } else if (ncases > 0) {
-    finalize_dt_batch<<<(ncases + 127) / 128, 128, 0, st>>>(args, ccs, ncases, nstages);
+    launch_dep(true, st, (ncases + 127) / 128, 128, finalize_dt_batch, args, ccs, ncases, nstages);
   }
 }
 
-void launch_step_begin_batch(const StageArgs *args, int ncases, int nstages, cudaStream_t st) {
-  step_begin_batch<<<(ncases + 127) / 128, 128, 0, st>>>(args, ncases, nstages);
-}
-
-// set the abort-order phase base of the current step (8 x step index)
-__global__ void set_phase_base_kernel(int *phase_base, int value, int fold) {
-  phase_base[0] = value;
-  phase_base[1] = fold;
-}
-void launch_set_phase_base(int *phase_base, int value, int fold, cudaStream_t st) {
-  set_phase_base_kernel<<<1, 1, 0, st>>>(phase_base, value, fold);
+void launch_batch_step(int *counters, const StageArgs *args, int ncases, int nstages,
+                       cudaStream_t st) {
+  launch_dep(false, st, 1, 128, batch_step_kernel, counters, args, ncases, nstages);
 }
 #endif
 

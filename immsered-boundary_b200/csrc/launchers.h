@@ -58,7 +58,20 @@ void launch_stage_batch(const StageArgs *args, const CaseConst *ccs, const int2 
 int batch_table_reserve(int device, int bytes);
 void batch_table_release(int device, int offset);
 cudaError_t batch_table_write(int offset, const void *src, int bytes);
-void launch_set_phase_base(int *phase_base, int value, int fold, cudaStream_t st);
+// a batched step: its first launch (counters: five ints, see the kernel),
+// then the cases' fills and viscous pass, blocks of kBatchBlock entries each
+// (launch_ib_batch: false, and nothing launched, when a case has more cells
+// than one CTA takes)
+void launch_batch_step(int *counters, const StageArgs *args, int ncases, int nstages,
+                       cudaStream_t st);
+void launch_pairs_batch(const BatchPairs *segs, const CaseConst *ccs, const int2 *blocks,
+                        int nblocks, bool prolong, cudaStream_t st);
+void launch_bc_batch(const BatchBc *segs, const CaseConst *ccs, const int2 *blocks, int nblocks,
+                     cudaStream_t st);
+bool launch_ib_batch(const BatchIb *segs, const CaseConst *ccs, int ncases, int most,
+                     cudaStream_t st);
+void launch_viscous_batch(const StageArgs *args, const CaseConst *ccs, const int2 *work, int nwork,
+                          int nstages, bool mixed, cudaStream_t st);
 void launch_take_folded_batch(const StageArgs *args, const CaseConst *ccs, int ncases, int nstages,
                               cudaStream_t st);
 // CFL pass over the work list's tiles, then dt of the first ncases cases, or
@@ -66,7 +79,6 @@ void launch_take_folded_batch(const StageArgs *args, const CaseConst *ccs, int n
 void launch_cfl_batch(const StageArgs *args, const CaseConst *ccs, const int2 *work, int nwork,
                       int nstages, const int *phase_base, int ncases, int grid, cudaStream_t st,
                       const int *case_list = nullptr);
-void launch_step_begin_batch(const StageArgs *args, int ncases, int nstages, cudaStream_t st);
 }  // namespace fast
 
 #undef IBGPU_DECLARE_LAUNCHERS

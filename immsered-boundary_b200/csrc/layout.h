@@ -166,6 +166,23 @@ struct IbArgs {
   const int *phase_base;
 };
 
+constexpr int kBatchBlock = 128;  // entries per block of a batched fill
+
+// Lists of a batch: case c's arguments of one launch; a batched launch runs
+// blocks (x: which of these, y: first entry) of several cases together.
+struct BatchPairs {
+  PairArgs a;
+  int c;
+};
+struct BatchBc {
+  BcArgs a;
+  int c;
+};
+struct BatchIb {
+  IbArgs a;
+  int c;
+};
+
 struct ForceArgs {
   const int32_t *body;   // per patch
   const int32_t *intp;   // 8 slots per patch
