@@ -10,6 +10,15 @@
 namespace ibgpu {
 namespace IBGPU_KNS {
 
+// threads of a viscous CTA: the FP64 build adds a ninth warp for the edge
+template <typename R>
+constexpr int visc_threads() {
+#ifdef IBGPU_FAST_BUILD
+  if (sizeof(R) == 8) return kTileCells + 32;
+#endif
+  return kTileCells;
+}
+
 // ---- coarse/fine interface ----------------------------------------------
 
 // AMR::InterfaceRestriction -> PairRestriction_2d -> AverageCell_2d
@@ -363,11 +372,75 @@ __global__ void __launch_bounds__(256) force_sum_kernel(ForceArgs a, CaseConst c
 }
 
 // ---- viscous face flux (NS_Solver::ComptViscousStress) -------------------
+// u, v, T of the tile and a one-cell halo (corners included) into the 18 x 18
+// region, zeros and flag 0 where no cell is: a thread per own cell, the last
+// four of the CTA's warps one side (lanes 0..15) and one corner (lane 16:
+// south-west, north-east, north-west, south-east) each.  Waits for the
+// previous kernel after the lookups that no step changes.  Returns the flags
+// of the thread's own cell.
+template <typename R, int NT, typename A>
+__device__ __forceinline__ uint8_t visc_region(const A &a, int tile, R *su, R *sv, R *sT,
+                                               uint8_t *sfl) {
+  constexpr int G = kTile + 2;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool own = tid < kTileCells;
+  const int rc = (((tid >> 4) & 15) + 1) * G + (tid & 15) + 1;
+  const int side = NT / 32 - 1 - (tid >> 5);
+  const bool halo = side < 4 && lane <= 16;
+  int nb = -1, hoff = 0, hr = 0;
+  if (halo) {
+    int x, y;  // position relative to the tile
+    if (lane < 16) {
+      x = side < 2 ? lane : (side == 2 ? -1 : kTile);
+      y = side < 2 ? (side ? kTile : -1) : lane;
+    } else {
+      x = side == 0 || side == 2 ? -1 : kTile;
+      y = side == 0 || side == 3 ? -1 : kTile;
+    }
+    const int ox = x < 0 ? -1 : (x >= kTile ? 1 : 0), oy = y < 0 ? -1 : (y >= kTile ? 1 : 0);
+    nb = a.tile_nb[(int64_t)tile * 9 + (oy + 1) * 3 + ox + 1];
+    hoff = (y - oy * kTile) * kTile + x - ox * kTile;
+    hr = (y + 1) * G + x + 1;
+  }
+  const int64_t os = (int64_t)tile * kTileCells + (own ? tid : 0);
+  const uint8_t fown = own ? a.flags[os] : (uint8_t)0;
+  const int64_t hs = (int64_t)nb * kTileCells + hoff;
+  const uint8_t fh = nb >= 0 ? a.flags[hs] : (uint8_t)0;
+  dep_wait();
+  R u = R(0), v = R(0), T = R(0), hu = R(0), hv = R(0), hT = R(0);
+  if (fown & CF_PRESENT) {
+    u = (R)a.s0[F_U][os];
+    v = (R)a.s0[F_V][os];
+    T = (R)a.s0[F_T][os];
+  }
+  if (fh & CF_PRESENT) {
+    hu = (R)a.s0[F_U][hs];
+    hv = (R)a.s0[F_V][hs];
+    hT = (R)a.s0[F_T][hs];
+  }
+  if (own) {
+    su[rc] = u;
+    sv[rc] = v;
+    sT[rc] = T;
+    sfl[rc] = fown;
+  }
+  if (halo) {
+    su[hr] = hu;
+    sv[hr] = hv;
+    sT[hr] = hT;
+    sfl[hr] = fh;
+  }
+  return fown;
+}
+
+// Expression by expression the reference: the exact build, and the mixed
+// build's FP32 (whose contractions and order of summation decide roundings of
+// its FP32 stage buffers, so it keeps them).
 // One tile per CTA: u, v, T of the tile and a one-cell halo (corners
 // included), every x- and y-face viscous flux into shared memory, then each
 // leaf cell's frozen residual parts vs(high) - vs(low) per direction.
 template <typename R, typename A>
-__device__ __forceinline__ void viscous_tile(const A &a, const CaseConst &cc, int tile) {
+__device__ __forceinline__ void viscous_tile_plain(const A &a, const CaseConst &cc, int tile) {
   constexpr int H = 1, G = kTile + 2 * H;  // 18
   __shared__ R su[G * G], sv[G * G], sT[G * G];
   __shared__ uint8_t sfl[G * G];
@@ -375,28 +448,7 @@ __device__ __forceinline__ void viscous_tile(const A &a, const CaseConst &cc, in
   __shared__ R vy[3][kYFaces];
   const int tid = threadIdx.x;
   const LevelConst &L = cc.lev[a.tile_level[tile]];
-  dep_wait();
-  for (int r = tid; r < G * G; r += kTileCells) {
-    int rx = r % G - H, ry = r / G - H;
-    int ox = rx < 0 ? -1 : (rx >= kTile ? 1 : 0);
-    int oy = ry < 0 ? -1 : (ry >= kTile ? 1 : 0);
-    uint8_t f = 0;
-    R u = R(0), v = R(0), T = R(0);
-    int nb = a.tile_nb[tile * 9 + (oy + 1) * 3 + (ox + 1)];
-    if (nb >= 0) {
-      int64_t s = (int64_t)nb * kTileCells + (ry - oy * kTile) * kTile + (rx - ox * kTile);
-      f = a.flags[s];
-      if (f & CF_PRESENT) {
-        u = (R)a.s0[F_U][s];
-        v = (R)a.s0[F_V][s];
-        T = (R)a.s0[F_T][s];
-      }
-    }
-    sfl[r] = f;
-    su[r] = u;
-    sv[r] = v;
-    sT[r] = T;
-  }
+  visc_region<R, kTileCells>(a, tile, su, sv, sT, sfl);
   __syncthreads();
   const R ikx = (R)L.inv_dx, iky = (R)L.inv_dy;
   const R Re = (R)cc.Re, S = (R)cc.s_over_t, qk = (R)cc.qk;
@@ -471,20 +523,108 @@ __device__ __forceinline__ void viscous_tile(const A &a, const CaseConst &cc, in
     const int xlo = ly * (kTile + 1) + lx, xhi = xlo + 1;
     const int ylo = ly * kTile + lx, yhi = ylo + kTile;
     double *vsd = const_cast<double *>(a.vsd);  // a stage's arguments only read it
-    vsd[0 * a.nslots + slot] = 0.0 - 0.0;
-    vsd[4 * a.nslots + slot] = 0.0 - 0.0;
+    // planes of x and y parts: the exact build has the mass's zeros too
+    constexpr int x0 = sizeof(R) == 8 ? 1 : 0, y0 = sizeof(R) == 8 ? 5 : 3;
+    if (sizeof(R) == 8) {
+      vsd[0 * a.nslots + slot] = 0.0 - 0.0;
+      vsd[4 * a.nslots + slot] = 0.0 - 0.0;
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      vsd[(int64_t)(1 + c) * a.nslots + slot] = (double)vx[c][xhi] - (double)vx[c][xlo];
-      vsd[(int64_t)(5 + c) * a.nslots + slot] = (double)vy[c][yhi] - (double)vy[c][ylo];
+      vsd[(int64_t)(x0 + c) * a.nslots + slot] = (double)vx[c][xhi] - (double)vx[c][xlo];
+      vsd[(int64_t)(y0 + c) * a.nslots + slot] = (double)vy[c][yhi] - (double)vy[c][ylo];
     }
   }
 }
 
+#ifdef IBGPU_FAST_BUILD
+// The FP64 build's face: T^1.5 as T^2 times the inverse root, one reciprocal
+// instead of the five divisions and the root (each some twenty FP64
+// instructions), the normal stress along the face only.  n: the normal
+// velocity component, t: the tangential one (the flux is the same in both
+// directions with the components' roles exchanged).
+__device__ __forceinline__ void viscous_face_fast(const CaseConst &cc, double area, double ikn,
+                                                  double ikt, double nL, double nR, double tL,
+                                                  double tR, double TL, double TR, double tn,
+                                                  double tt, double &fn, double &ft, double &fe) {
+  typedef FastMath<double> M;
+  const double T = 0.5 * (TL + TR);
+  const double T2 = T * T;  // (T = 0 has no viscosity, not 0 times an infinite root)
+  const double mu = (T2 == 0.0 ? 0.0 : T2 * M::rsqrt(T)) * ((1.0 + cc.s_over_t) * M::rcp(T + cc.s_over_t)) * area;
+  const double dn_n = (nR - nL) * ikn, dt_n = (tR - tL) * ikn;      // normal derivatives
+  const double kt = 0.25 * ikt;
+  const double dn_t = tn * kt, dt_t = tt * kt;                      // tangential derivatives
+  const double m = mu * cc.inv_Re;
+  fn = (m * (2.0 / 3.0)) * fma(2.0, dn_n, -dt_t);
+  ft = m * (dn_t + dt_n);
+  fe = fma(0.5 * (nL + nR), fn, fma(0.5 * (tL + tR), ft, (cc.qk * mu) * ((TR - TL) * ikn)));
+}
+
+// The FP64 build's tile: a thread per cell (its west and south face), a ninth
+// warp for the east and north faces, whole warps for the halo sides (288
+// threads); one frozen residual per component, the x and y parts added: 24
+// bytes a cell written here and read by every stage instead of 64.  With the
+// divisions gone it is bound by one load round trip per tile.  16 steps of
+// the 914 k-row nested mesh 2.32 -> 1.96 ms, 24 of the airfoil 1.06 -> 0.92.
+template <typename A>
+__device__ __forceinline__ void viscous_tile_fp64(const A &a, const CaseConst &cc, int tile) {
+  constexpr int G = kTile + 2, kFX = kTile + 1, NF = kTile * kFX;
+  __shared__ double su[G * G], sv[G * G], sT[G * G];
+  __shared__ uint8_t sfl[G * G];
+  __shared__ double vx[3][NF];  // x-face i of row j at j*17 + i: x-mom, y-mom, energy
+  __shared__ double vy[3][NF];  // y-face j of column i at j*16 + i
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool own = tid < kTileCells;
+  const int tx = tid & 15, ty = (tid >> 4) & 15;
+  const LevelConst &L = cc.lev[a.tile_level[tile]];
+  const int rc = (ty + 1) * G + tx + 1;
+  const uint8_t fown = visc_region<double, kTileCells + 32>(a, tile, su, sv, sT, sfl);
+  __syncthreads();
+  const double ikx = L.inv_dx, iky = L.inv_dy, ax = L.area_x, ay = L.area_y;
+  // face between region cells l and l + step, tangential step ts
+  auto face = [&](bool xdir, int l, double *out, int at) {
+    const int step = xdir ? 1 : G, ts = xdir ? G : 1, r = l + step;
+    double f[3] = {0.0, 0.0, 0.0};
+    if ((sfl[l] & CF_PRESENT) && (sfl[r] & CF_PRESENT) && ((sfl[l] | sfl[r]) & CF_NORMAL)) {
+      const double tu = su[l + ts] + su[r + ts] - su[l - ts] - su[r - ts],
+              tv = sv[l + ts] + sv[r + ts] - sv[l - ts] - sv[r - ts];
+      const double *n = xdir ? su : sv, *t = xdir ? sv : su;
+      viscous_face_fast(cc, xdir ? ax : ay, xdir ? ikx : iky, xdir ? iky : ikx, n[l], n[r], t[l],
+                        t[r], sT[l], sT[r], xdir ? tu : tv, xdir ? tv : tu, f[xdir ? 0 : 1],
+                        f[xdir ? 1 : 0], f[2]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[c * NF + at] = f[c];
+  };
+  if (own) {
+    face(true, rc - 1, &vx[0][0], ty * kFX + tx);
+    face(false, rc - G, &vy[0][0], ty * kTile + tx);
+  } else if (lane < 16) {
+    face(true, (lane + 1) * G + kTile, &vx[0][0], lane * kFX + kTile);
+  } else {
+    face(false, kTile * G + (lane & 15) + 1, &vy[0][0], kTile * kTile + (lane & 15));
+  }
+  __syncthreads();
+  if (own && (fown & CF_NORMAL)) {
+    double *vsd = const_cast<double *>(a.vsd);  // a stage's arguments only read it
+    const int x = ty * kFX + tx, y = ty * kTile + tx;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      vsd[(int64_t)c * a.nslots + (int64_t)tile * kTileCells + tid] =
+          (vx[c][x + 1] - vx[c][x]) + (vy[c][y + kTile] - vy[c][y]);
+  }
+}
+#endif
+
 template <typename R>
-__global__ void __launch_bounds__(kTileCells) viscous_kernel(ViscArgs a, CaseConst cc) {
+__global__ void __launch_bounds__(visc_threads<R>()) viscous_kernel(ViscArgs a, CaseConst cc) {
   dep_begin();
-  viscous_tile<R>(a, cc, a.tile_begin + (int)blockIdx.x);
+  const int tile = a.tile_begin + (int)blockIdx.x;
+#ifdef IBGPU_FAST_BUILD
+  if constexpr (sizeof(R) == 8) viscous_tile_fp64(a, cc, tile);
+  else
+#endif
+    viscous_tile_plain<R>(a, cc, tile);
 }
 
 #ifdef IBGPU_FAST_BUILD
@@ -529,12 +669,13 @@ __global__ void __launch_bounds__(kIbBlock)
   if (i < s.a.n) ib_put(s.a, i, o);
 }
 template <typename R>
-__global__ void __launch_bounds__(kTileCells)
+__global__ void __launch_bounds__(visc_threads<R>())
     viscous_kernel_batch(const StageArgs *__restrict__ args, const CaseConst *__restrict__ ccs,
                          const int2 *__restrict__ work, int nstages) {
   dep_begin();
   const int2 it = work[blockIdx.x];
-  viscous_tile<R>(args[it.x * nstages], ccs[it.x], it.y);
+  if constexpr (sizeof(R) == 8) viscous_tile_fp64(args[it.x * nstages], ccs[it.x], it.y);
+  else viscous_tile_plain<R>(args[it.x * nstages], ccs[it.x], it.y);
 }
 
 void launch_pairs_batch(const BatchPairs *segs, const CaseConst *ccs, const int2 *blocks,
@@ -556,8 +697,8 @@ bool launch_ib_batch(const BatchIb *segs, const CaseConst *ccs, int ncases, int 
 void launch_viscous_batch(const StageArgs *args, const CaseConst *ccs, const int2 *work, int nwork,
                           int nstages, bool mixed, cudaStream_t st) {
   if (nwork <= 0) return;
-  if (mixed) launch_dep(true, st, nwork, kTileCells, viscous_kernel_batch<float>, args, ccs, work, nstages);
-  else launch_dep(true, st, nwork, kTileCells, viscous_kernel_batch<double>, args, ccs, work, nstages);
+  if (mixed) launch_dep(true, st, nwork, visc_threads<float>(), viscous_kernel_batch<float>, args, ccs, work, nstages);
+  else launch_dep(true, st, nwork, visc_threads<double>(), viscous_kernel_batch<double>, args, ccs, work, nstages);
 }
 #endif
 
@@ -590,11 +731,11 @@ void launch_viscous(const ViscArgs &a, const CaseConst &cc, int ntiles, bool mix
   if (ntiles <= 0) return;
 #ifdef IBGPU_FAST_BUILD
   if (mixed) {
-    launch_dep(dep, st, ntiles, kTileCells, viscous_kernel<float>, a, cc);
+    launch_dep(dep, st, ntiles, visc_threads<float>(), viscous_kernel<float>, a, cc);
     return;
   }
 #endif
-  launch_dep(dep, st, ntiles, kTileCells, viscous_kernel<double>, a, cc);
+  launch_dep(dep, st, ntiles, visc_threads<double>(), viscous_kernel<double>, a, cc);
 }
 
 }  // namespace IBGPU_KNS

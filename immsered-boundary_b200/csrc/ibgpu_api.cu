@@ -315,6 +315,7 @@ void fill_case_const(const ibgpu_case *cs, CaseConst &k) {
   k.inv_Rg = 1.0 / cs->Rg;
   k.gam_gm1 = k.gama / k.gm1;
   k.two_gama = 2.0 * k.gama;
+  k.inv_Re = 1.0 / cs->Re;
   k.Cp = cs->Cp;
   k.p_ref = cs->p_ref;
   k.area_ref = cs->area_ref;
@@ -725,7 +726,10 @@ int ibgpu_upload_topology(ibgpu_ctx *ctx, const ibgpu_cells *cells) {
   for (int b = 0; b < 2; ++b)
     for (int f = 0; f < 4; ++f)
       if ((rc = keep_alloc(ctx, (unsigned char **)&ctx->d_buf[b][f], (size_t)nslots * buf_elem))) return rc;
-  if (cs.viscous && (rc = keep_alloc(ctx, &ctx->d_vsd, (size_t)nslots * 8))) return rc;
+  // planes of the frozen viscous residual (StageArgs::vsd)
+  const size_t vplanes =
+      cs.precision == IBGPU_FP64_EXACT ? 8 : (cs.precision == IBGPU_MIXED ? 6 : 3);
+  if (cs.viscous && (rc = keep_alloc(ctx, &ctx->d_vsd, (size_t)nslots * vplanes))) return rc;
   cudaStream_t st = ctx->stream;
   CK(cudaMemcpyAsync(ctx->d_tile_nb, h_nb.data(), h_nb.size() * 4, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->d_tile_level, h_tile_level.data(), ntiles * 4, cudaMemcpyHostToDevice, st));
@@ -768,7 +772,7 @@ int ibgpu_upload_topology(ibgpu_ctx *ctx, const ibgpu_cells *cells) {
   for (int f = 0; f < kStateFields; ++f) CK(cudaMemsetAsync(ctx->d_s0[f], 0, nslots * 8, st));
   for (int b = 0; b < 2; ++b)
     for (int f = 0; f < 4; ++f) CK(cudaMemsetAsync(ctx->d_buf[b][f], 0, nslots * buf_elem, st));
-  if (ctx->d_vsd) CK(cudaMemsetAsync(ctx->d_vsd, 0, nslots * 8 * 8, st));
+  if (ctx->d_vsd) CK(cudaMemsetAsync(ctx->d_vsd, 0, nslots * vplanes * sizeof(double), st));
   CK(cudaStreamSynchronize(st));
   ctx->tilemap = std::move(tilemap);
   // each row's layout bits, against which ibgpu_update_flags checks new flags

@@ -684,11 +684,13 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
       } else {
         double sx = (sizeof(R) == 4) ? (double)(sxl[c] - sxh[c]) : (double)sxl[c] - (double)sxh[c];
         double sy = (sizeof(R) == 4) ? (double)(syl[c] - syh[c]) : (double)syl[c] - (double)syh[c];
-        if (VISC) {
-          sx += a.vsd[(int64_t)c * a.nslots + slot];
-          sy += a.vsd[(int64_t)(4 + c) * a.nslots + slot];
+        // frozen viscous residual of the momenta and the energy
+        if (VISC && c > 0 && sizeof(R) == 4) {
+          sx += a.vsd[(int64_t)(c - 1) * a.nslots + slot];
+          sy += a.vsd[(int64_t)(2 + c) * a.nslots + slot];
         }
         res[c] = sx + sy;
+        if (VISC && c > 0 && sizeof(R) == 8) res[c] += a.vsd[(int64_t)(c - 1) * a.nslots + slot];
       }
     }
     const double dt = a.diag->dt;

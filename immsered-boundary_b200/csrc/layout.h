@@ -45,7 +45,7 @@ struct LevelConst {
 struct CaseConst {
   double gama, Rg, Cv, Ma, Re, qk, s_over_t, dt_ratio;
   double gm1, gamaRg, inv_Rg, Cp;
-  double gam_gm1, two_gama;  // gama / (gama - 1), 2 gama (fast builds)
+  double gam_gm1, two_gama, inv_Re;  // gama / (gama - 1), 2 gama, 1 / Re (fast builds)
   double p_ref, area_ref, shear_ref, L_ref, mu;
   double initvar[7];
   LevelConst lev[kMaxLevels];
@@ -102,7 +102,10 @@ struct StageArgs {
   const uint8_t *tile_uniform;  // 1: tile and side neighbours all recovering leaf cells
   const uint8_t *flags;
   double *s0[kStateFields];  // step state rho u v p e T
-  const double *vsd;         // frozen viscous residual parts [8][nslots] or null
+  // frozen viscous residual or null: FP64 [3][nslots] (x-momentum,
+  // y-momentum, energy), mixed the x parts [3] and y parts [3], exact build
+  // the x parts [4] and y parts [4] (mass too)
+  const double *vsd;
   int64_t nslots;
   DevDiag *diag;
   int tile_begin;
