@@ -1485,12 +1485,12 @@ struct ibgpu_batch {
   // the fills of the cases that are due at ts % full_period == q, one launch
   // after another: blocks of the segments below
   struct Fill {
-    int kind;  // 0 restriction, 1 prolongation, 2 domain ghosts
-    int2 *blocks;
+    int kind;      // 0 restriction, 1 prolongation, 2 domain ghosts
+    size_t first;  // blocks [first, first + n) of d_fill_blocks
     int n;
   };
   std::vector<std::vector<Fill>> fills;
-  std::vector<int2 *> fill_blocks;  // owned (several phases share one)
+  int2 *d_fill_blocks = nullptr;  // every phase's (phases share equal lists)
   BatchPairs *d_pairs = nullptr;
   BatchBc *d_bcs = nullptr;
   BatchIb *d_ibs = nullptr;
@@ -1529,8 +1529,8 @@ struct ibgpu_batch {
   }
   void release() {
     drop_graphs();
-    for (auto w : fill_blocks) cudaFree(w);
-    fill_blocks.clear();
+    cudaFree(d_fill_blocks);
+    d_fill_blocks = nullptr;
     fills.clear();
     cudaFree(d_pairs);
     cudaFree(d_bcs);
@@ -1721,8 +1721,8 @@ int enqueue_batch_step(ibgpu_batch *b, int q, int cfl, cudaStream_t st) {
   auto run_fills = [&](bool domain) -> int {
     for (const auto &f : b->fills[q]) {
       if ((f.kind == 2) != domain) continue;
-      if (domain) fast::launch_bc_batch(b->d_bcs, b->d_ccs, f.blocks, f.n, st);
-      else fast::launch_pairs_batch(b->d_pairs, b->d_ccs, f.blocks, f.n, f.kind == 1, st);
+      if (domain) fast::launch_bc_batch(b->d_bcs, b->d_ccs, b->d_fill_blocks + f.first, f.n, st);
+      else fast::launch_pairs_batch(b->d_pairs, b->d_ccs, b->d_fill_blocks + f.first, f.n, f.kind == 1, st);
       CK(cudaGetLastError());
     }
     return IBGPU_OK;
@@ -1752,7 +1752,8 @@ int build_fills(ibgpu_batch *b) {
   std::vector<BatchBc> bcs;
   std::vector<BatchIb> ibs;
   std::map<std::vector<int>, int> known;         // (kind, case, l0, l1 | wave) -> segment
-  std::map<std::vector<int>, int2 *> block_list;  // segments -> their blocks
+  std::map<std::vector<int>, std::pair<size_t, int>> block_list;  // segments -> their blocks
+  std::vector<int2> blocks;
   const int n = (int)b->cases.size();
   b->fills.assign(b->full_period, {});
   for (int i = 0; i < n; ++i) {
@@ -1799,27 +1800,23 @@ int build_fills(ibgpu_batch *b) {
       }
       for (const auto &round : rounds) {
         std::vector<int> key{kind};
-        std::vector<int2> blocks;
-        for (const auto &s : round) {
-          key.push_back(s[0]);
-          for (int f = s[1]; f < s[2]; f += kBatchBlock) blocks.push_back(make_int2(s[0], f));
+        for (const auto &g : round) key.push_back(g[0]);
+        auto it = block_list.emplace(key, std::make_pair(blocks.size(), 0));
+        if (it.second) {
+          for (const auto &g : round)
+            for (int f = g[1]; f < g[2]; f += kBatchBlock) blocks.push_back(make_int2(g[0], f));
+          it.first->second.second = (int)(blocks.size() - it.first->second.first);
         }
-        int2 *&d = block_list[key];
-        if (!d) {
-          int rc = dev_alloc(&d, blocks.size());
-          if (rc) return rc;
-          b->fill_blocks.push_back(d);
-          CK(cudaMemcpy(d, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice));
-        }
-        b->fills[q].push_back({kind, d, (int)blocks.size()});
+        b->fills[q].push_back({kind, it.first->second.first, it.first->second.second});
       }
     }
   }
   b->n_ibs = (int)ibs.size();
   int rc;
   if ((rc = dev_alloc(&b->d_pairs, pairs.size())) || (rc = dev_alloc(&b->d_bcs, bcs.size())) ||
-      (rc = dev_alloc(&b->d_ibs, ibs.size())))
+      (rc = dev_alloc(&b->d_ibs, ibs.size())) || (rc = dev_alloc(&b->d_fill_blocks, blocks.size())))
     return rc;
+  CK(cudaMemcpy(b->d_fill_blocks, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b->d_pairs, pairs.data(), pairs.size() * sizeof(BatchPairs), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b->d_bcs, bcs.data(), bcs.size() * sizeof(BatchBc), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b->d_ibs, ibs.data(), ibs.size() * sizeof(BatchIb), cudaMemcpyHostToDevice));

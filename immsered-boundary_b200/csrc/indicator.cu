@@ -15,12 +15,14 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "../../include/ibgpu.h"
+#include "dependent.cuh"
 #include "host_internal.h"
 #include "layout.h"
 #include "tcgen05.cuh"
@@ -33,7 +35,15 @@ constexpr int kHid = IBGPU_MLP_HIDDEN;    // 64
 constexpr int kOut = IBGPU_MLP_CLASSES;   // 3
 constexpr int kRows = 128;                // rows per tile = M of every MMA
 constexpr int kThreads = 128;
+constexpr int kFwdCtas = 4;               // resident inference CTAs per SM
 constexpr int kOnesRow = kIn;             // feature held at 1 in the training tiles (bias gradients)
+
+// K-slab pitches of the operand tiles (8 bf16 columns of every row): 16 bytes
+// over rows x 16, so that the 16-byte pieces of one row (consecutive in
+// memory, hence loaded by consecutive lanes) land in different banks
+constexpr int kXPitch = kRows * 16 + 16;  // feature tile
+constexpr int kWPitch = kHid * 16 + 16;   // weight tiles
+constexpr int kInSlabs = kIn / 8;         // 14
 
 // parameter array offsets (floats)
 constexpr int P_W1 = 0;
@@ -49,7 +59,7 @@ static_assert(P_COUNT == IBGPU_MLP_PARAMS, "parameter layout");
 constexpr uint32_t T_D1 = 0;      // layer-1 pre-activation   (64)
 constexpr uint32_t T_D2 = 64;     // layer-2 pre-activation   (64)
 constexpr uint32_t T_COLS_TRAIN = 512;
-constexpr uint32_t T_COLS_FWD = 256;
+constexpr uint32_t T_COLS_FWD = 128;
 
 constexpr long long kWaitCycles = 2000000000ll;  // ~1 s at the boost clock
 
@@ -76,47 +86,55 @@ __device__ __forceinline__ float tanh_sfu(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu(float z) {
-  const float u = kGeluA * (z + kGeluB * z * z * z);
-  return 0.5f * z * (1.0f + tanh_sfu(u));
+// Two elements at a time: the paired FP32 instructions (f32x2) halve the issue
+// slots of the epilogues, which bound these kernels.
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 gelu2(float2 z) {
+  const float2 c = __fmul2_rn(__fmul2_rn(f2(kGeluB), z), z);
+  const float2 u = __fmul2_rn(f2(kGeluA), __ffma2_rn(c, z, z));
+  const float2 th = make_float2(tanh_sfu(u.x), tanh_sfu(u.y));
+  return __fmul2_rn(__fmul2_rn(f2(0.5f), z), __fadd2_rn(f2(1.0f), th));
 }
 // GELU and its derivative d/dz [0.5 z (1 + tanh u)], u = a (z + b z^3)
-__device__ __forceinline__ void gelu_and_grad(float z, float &g, float &gp) {
-  const float u = kGeluA * (z + kGeluB * z * z * z);
-  const float th = tanh_sfu(u);
-  g = 0.5f * z * (1.0f + th);
-  gp = 0.5f * (1.0f + th) + 0.5f * z * (1.0f - th * th) * kGeluA * (1.0f + 3.0f * kGeluB * z * z);
-}
-
-__device__ __forceinline__ void st_bf16(uint8_t *base, int off, float v) {
-  *reinterpret_cast<uint16_t *>(base + off) = bf16_bits(v);
+__device__ __forceinline__ void gelu_and_grad2(float2 z, float2 &g, float2 &gp) {
+  const float2 c = __fmul2_rn(__fmul2_rn(f2(kGeluB), z), z);
+  const float2 u = __fmul2_rn(f2(kGeluA), __ffma2_rn(c, z, z));
+  const float2 th = make_float2(tanh_sfu(u.x), tanh_sfu(u.y));
+  const float2 nt = make_float2(-th.x, -th.y);
+  const float2 h = __fmul2_rn(f2(0.5f), z), s = __fadd2_rn(f2(1.0f), th);
+  g = __fmul2_rn(h, s);
+  const float2 d = __fmul2_rn(__fmul2_rn(h, __ffma2_rn(nt, th, f2(1.0f))), f2(kGeluA));
+  const float2 w = __ffma2_rn(__fmul2_rn(f2(3.0f * kGeluB), z), z, f2(1.0f));
+  gp = __ffma2_rn(f2(0.5f), s, __fmul2_rn(d, w));
 }
 
 // ---------------------------------------------------------------------------
-// Training kernel: 256 threads, two per tile row.  Warp w reads Tensor
+// Training kernel: 512 threads, four per tile row.  Warp w reads Tensor
 // Memory lane quarter w % 4 (tile rows 32 (w % 4) ..) and owns accumulator
-// columns [32 (w / 4), +32) of the 64-wide layers.  Every activation and
+// columns [16 (w / 4), +16) of the 64-wide layers.  Every activation and
 // gradient tile is stored once, row-major in the K-major layout (8-column
 // slabs of 2048 bytes); the weight-gradient products read those same tiles
 // as MN-major operands of their transposes, so nothing is transposed in
 // shared memory.  Shared memory (bytes):
-constexpr int kThreadsTrain = 256;
+constexpr int kThreadsTrain = 512;
+constexpr int kCols = kHid / (kThreadsTrain / kRows);  // columns per thread
 constexpr int kSlab = kRows * 16;  // 8 bf16 columns of a 128-row tile
 struct TrainSmem {
   // X of two tiles (the next one is stored while the weight gradients of
   // the current one still read it): 16 slabs, features 112 = 1 (bias rows
   // of the weight gradients) and 113..127 = 0
   static constexpr int X0 = 0;
-  static constexpr int X1 = X0 + 16 * kSlab;
-  static constexpr int H = X1 + 16 * kSlab;    // [h1 | h2], 16 slabs
+  static constexpr int X1 = X0 + 16 * kXPitch;
+  static constexpr int H = X1 + 16 * kXPitch;    // [h1 | h2], 16 slabs
   static constexpr int DZ = H + 16 * kSlab;    // [dz1 | dz2 | dz3 (16 columns)], 18 slabs
   static constexpr int W1 = DZ + 18 * kSlab;   // [64 x 112] B of layer 1
-  static constexpr int W2 = W1 + kHid * kIn * 2;       // [64 x 64]  B of layer 2
-  static constexpr int W2T = W2 + kHid * kHid * 2;     // [64 x 64]  B of dh1
-  static constexpr int BIAS = W2T + kHid * kHid * 2;   // b1, b2, b3 (f32)
-  static constexpr int W3F = BIAS + 1024;              // W3 rounded to bf16, as f32 [3 x 64]
-  static constexpr int XCH = W3F + 1024;               // row exchange between column halves [128 x 4] f32
-  static constexpr int BYTES = XCH + kRows * 16;
+  static constexpr int W2 = W1 + kInSlabs * kWPitch;        // [64 x 64]  B of layer 2
+  static constexpr int W2T = W2 + kHid / 8 * kWPitch;       // [64 x 64]  B of dh1
+  static constexpr int BIAS = W2T + kHid / 8 * kWPitch;   // b1, b2, b3 (f32)
+  static constexpr int W3F = BIAS + 544;               // W3 rounded to bf16, as f32 [3 x 64]
+  static constexpr int W3R = W3F + 768;                // the same [64 x 4]
+  static constexpr int XCH = W3R + 1024;               // row exchange between column groups [4 x 128 x 4] f32
+  static constexpr int BYTES = XCH + 4 * kRows * 16;
 };
 static_assert(TrainSmem::BYTES <= 227 * 1024, "shared memory budget");
 
@@ -127,33 +145,88 @@ constexpr uint32_t TT_GCAT = 128;  // [h1|h2]^T [dz2|dz3], accumulated         (
 constexpr uint32_t TT_G1 = 208;    // [x|1]^T [dz1|dz2|dz3], accumulated      (144)
 static_assert(TT_G1 + 144 <= T_COLS_TRAIN, "tensor memory budget");
 
+// Inference kernels: h1 takes X's place once the layer-1 MMAs have read it,
+// so that four CTAs share an SM (shared memory and Tensor Memory: 128 columns
+// each).
 struct FwdSmem {
   static constexpr int X = 0;
-  static constexpr int H1 = X + kRows * kIn * 2;
-  static constexpr int W1 = H1 + kRows * kHid * 2;
-  static constexpr int W2 = W1 + kHid * kIn * 2;
-  static constexpr int BIAS = W2 + kHid * kHid * 2;
-  static constexpr int W3F = BIAS + 1024;  // W3 rounded to bf16, as f32 [3 x 64]
-  static constexpr int BYTES = W3F + 1024;
+  static constexpr int H1 = X;
+  static constexpr int W1 = X + kInSlabs * kXPitch;
+  static constexpr int W2 = W1 + kInSlabs * kWPitch;
+  static constexpr int BIAS = W2 + kHid / 8 * kWPitch;
+  static constexpr int W3R = BIAS + 544;  // W3 rounded to bf16, as f32 [64 x 4]
+  static constexpr int BYTES = W3R + 1024;
 };
 
-// Weights (rounded to bf16) into their B-operand tiles; W3 (3 rows, used
-// on the CUDA cores) rounded to bf16 and kept as f32; biases as f32.
-__device__ void load_weights(const float *__restrict__ P, uint8_t *sW1, uint8_t *sW2,
-                             uint8_t *sW2T, float *sB, float *sW3f) {
-  using tc::kmajor_off;
-  for (int i = threadIdx.x; i < kHid * kIn; i += blockDim.x) {
-    const int o = i / kIn, k = i % kIn;
-    st_bf16(sW1, kmajor_off(kHid, o, k), P[P_W1 + i]);
+// 8 consecutive weights of a row (2 loads where the array allows, else 8)
+__device__ __forceinline__ void load8(const float *__restrict__ p, bool vec, float (&v)[8]) {
+  if (vec) {
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = p[e];
   }
-  for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) {
-    const int o = i / kHid, k = i % kHid;
-    const float w = P[P_W2 + i];
-    st_bf16(sW2, kmajor_off(kHid, o, k), w);
-    if (sW2T) st_bf16(sW2T, kmajor_off(kHid, k, o), w);
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                    pack_bf16(v[6], v[7]));
+}
+
+// Weights (rounded to bf16) into their B-operand tiles, 16 bytes (8 columns of
+// a row) at a time, consecutive lanes on consecutive memory and every load of
+// a matrix before its first store (NT threads); W3 (3 rows, used on the CUDA
+// cores) rounded to bf16 and kept as f32 (by unit, and in training by row);
+// biases as f32.  One load after another, with a division and a two-byte
+// store per element, took most of a small call's time.
+template <int NT>
+__device__ __forceinline__ void load_weights(const float *__restrict__ P, uint8_t *sW1,
+                                             uint8_t *sW2, uint8_t *sW2T, float *sB, float *sW3f,
+                                             float4 *sW3r) {
+  const int t = threadIdx.x;
+  const bool vec = (reinterpret_cast<uintptr_t>(P) & 15u) == 0;
+  auto matrix = [&](const float *W, int cols, auto slabs, uint8_t *dst) {
+    constexpr int kSlabs = decltype(slabs)::value, kN = kHid * kSlabs;
+    constexpr int kIt = (kN + NT - 1) / NT;
+    float v[kIt][8];
+#pragma unroll
+    for (int k = 0; k < kIt; ++k) {
+      const int i = t + k * NT;
+      if (i < kN) load8(W + (i / kSlabs) * cols + 8 * (i % kSlabs), vec, v[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kIt; ++k) {
+      const int i = t + k * NT;
+      if (i < kN)
+        *reinterpret_cast<uint4 *>(dst + (i % kSlabs) * kWPitch + (i / kSlabs) * 16) = pack8(v[k]);
+    }
+  };
+  static_assert(P_W2 % 4 == 0 && kIn % 4 == 0, "16-byte rows");
+  matrix(P + P_W1, kIn, std::integral_constant<int, kIn / 8>(), sW1);
+  matrix(P + P_W2, kHid, std::integral_constant<int, kHid / 8>(), sW2);
+  if (sW2T) {
+    // transposed: row o takes column o of W2
+    for (int i = t; i < kHid * (kHid / 8); i += NT) {
+      const int o = i % kHid, k = i / kHid;
+      const float *q = P + P_W2 + 8 * k * kHid + o;
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = q[e * kHid];
+      *reinterpret_cast<uint4 *>(sW2T + k * kWPitch + o * 16) = pack8(v);
+    }
   }
-  for (int i = threadIdx.x; i < kOut * kHid; i += blockDim.x) sW3f[i] = bf16_round(P[P_W3 + i]);
-  for (int i = threadIdx.x; i < 2 * kHid + 4; i += blockDim.x) {
+  for (int i = t; i < kHid; i += NT) {
+    const float w0 = bf16_round(P[P_W3 + i]), w1 = bf16_round(P[P_W3 + kHid + i]),
+                w2 = bf16_round(P[P_W3 + 2 * kHid + i]);
+    sW3r[i] = make_float4(w0, w1, w2, 0.0f);
+    if (sW3f) {
+      sW3f[i] = w0;
+      sW3f[kHid + i] = w1;
+      sW3f[2 * kHid + i] = w2;
+    }
+  }
+  for (int i = t; i < 2 * kHid + 4; i += NT) {
     float b = 0.0f;
     if (i < kHid) b = P[P_B1 + i];
     else if (i < 2 * kHid) b = P[P_B2 + i - kHid];
@@ -192,43 +265,36 @@ __device__ __forceinline__ bool commit_and_wait(uint64_t *bar, uint32_t &phase, 
   return *(volatile int *)abort_flag == 0;
 }
 
-// 64 f32 columns of this thread's lane starting at `col`, plus bias.
-// (the four loads issued back to back, one wait)
-__device__ __forceinline__ void tmem_row64(uint32_t taddr, const float *bias, float (&v)[64]) {
-  uint32_t r[4][16];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) tc::tmem_ld16(taddr + 16 * q, r[q]);
+// 32 f32 columns of this thread's lane (two loads, one wait)
+__device__ __forceinline__ void tmem_row32(uint32_t taddr, float (&v)[32]) {
+  uint32_t r[2][16];
+  tc::tmem_ld16(taddr, r[0]);
+  tc::tmem_ld16(taddr + 16, r[1]);
   tc::tmem_wait_ld16(r[0]);
+  tc::tmem_tie16(r[1]);
 #pragma unroll
-  for (int q = 1; q < 4; ++q) tc::tmem_tie16(r[q]);
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int e = 0; e < 16; ++e) v[16 * q + e] = __uint_as_float(r[q][e]) + (bias ? bias[16 * q + e] : 0.0f);
+  for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e >> 4][e & 15]);
 }
 
-// Row-major [rows x 64] bf16 A tile: this thread's row from 64 values.
-__device__ __forceinline__ void store_row64(uint8_t *tile, int t, const float (&v)[64]) {
+// Feature rows of a tile -> X: the tile's rows are one run of 16-byte pieces
+// (14 per row), consecutive lanes take consecutive pieces.  (A lane per row,
+// 224 bytes apart, asked for 32 half-used sectors per load.)  Rows past n are
+// zero.
+__device__ __forceinline__ void load_x_tile(const uint16_t *__restrict__ feat, int64_t tile,
+                                            int64_t n, int t, uint8_t *sX) {
+  const uint4 *src = reinterpret_cast<const uint4 *>(feat + tile * kRows * kIn);
+  const int64_t left = n - tile * kRows;
+  const int pieces = (int)(left < kRows ? left : kRows) * kInSlabs;
+  uint4 w[kInSlabs];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    uint4 w;
-    w.x = pack_bf16(v[8 * c + 0], v[8 * c + 1]);
-    w.y = pack_bf16(v[8 * c + 2], v[8 * c + 3]);
-    w.z = pack_bf16(v[8 * c + 4], v[8 * c + 5]);
-    w.w = pack_bf16(v[8 * c + 6], v[8 * c + 7]);
-    *reinterpret_cast<uint4 *>(tile + c * (kRows * 16) + t * 16) = w;
+  for (int k = 0; k < kInSlabs; ++k) {
+    const int i = t + k * kThreads;
+    w[k] = i < pieces ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
   }
-}
-
-// Feature row -> X (row-major A tile).
-__device__ __forceinline__ void load_x_row(const uint16_t *__restrict__ feat, int64_t row, bool valid,
-                                           int t, uint8_t *sX) {
-  const uint4 *src = reinterpret_cast<const uint4 *>(feat + row * kIn);
-#pragma unroll 2
-  for (int c = 0; c < kIn / 8; ++c) {
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (valid) w = __ldg(src + c);
-    *reinterpret_cast<uint4 *>(sX + c * (kRows * 16) + t * 16) = w;
+#pragma unroll
+  for (int k = 0; k < kInSlabs; ++k) {
+    const int i = t + k * kThreads;
+    *reinterpret_cast<uint4 *>(sX + (i % kInSlabs) * kXPitch + (i / kInSlabs) * 16) = w[k];
   }
 }
 
@@ -249,8 +315,13 @@ __device__ __forceinline__ void load_x_row(const uint16_t *__restrict__ feat, in
 // The unwaited weight-gradient MMAs overlap the next epilogue; the tile
 // buffers they read are rewritten only after a later commit covers them.
 // Products on the CUDA cores take bf16-rounded operands and accumulate in
-// f32, as the tensor core does.  (Two tiles in flight, alternating steps in
-// the same warps, measured slower: 116 us against 91 us for 262,144 rows.)
+// f32, as the tensor core does.  Bound by the latency of each tile's three
+// MMA round trips and the epilogues between them (tensor pipe 15 % busy, 33 %
+// of the issue slots): 262,144 rows 92 -> 81 us, 8,192 rows (one tile per
+// CTA) 18.8 -> 15.0 us with coalesced tile loads, batched weight loads and
+// paired FP32 epilogues; four threads per row instead of two changed nothing
+// by itself.  (Two tiles in flight, alternating steps in the same warps,
+// measured slower: 116 us against 91.)
 __device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t &phase, int *abort_flag) {
   const bool ok = tc::mbar_wait_bounded(bar, phase, kWaitCycles);
   if (ok) phase ^= 1u;
@@ -259,27 +330,24 @@ __device__ __forceinline__ bool wait_phase(uint64_t *bar, uint32_t &phase, int *
   return *(volatile int *)abort_flag == 0;
 }
 
-// 32 f32 columns of this thread's lane (two loads, one wait)
-__device__ __forceinline__ void tmem_row32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[2][16];
-  tc::tmem_ld16(taddr, r[0]);
-  tc::tmem_ld16(taddr + 16, r[1]);
-  tc::tmem_wait_ld16(r[0]);
-  tc::tmem_tie16(r[1]);
+// 16 f32 columns of this thread's lane
+__device__ __forceinline__ void tmem_row16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  tc::tmem_ld16(taddr, r);
+  tc::tmem_wait_ld16(r);
 #pragma unroll
-  for (int e = 0; e < 32; ++e) v[e] = __uint_as_float(r[e >> 4][e & 15]);
+  for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(r[e]);
 }
-__device__ __forceinline__ void tmem_store32(uint32_t taddr, const float (&v)[32]) {
-  uint32_t r[2][16];
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const float (&v)[16]) {
+  uint32_t r[16];
 #pragma unroll
-  for (int e = 0; e < 32; ++e) r[e >> 4][e & 15] = __float_as_uint(v[e]);
-  tc::tmem_st16(taddr, r[0]);
-  tc::tmem_st16(taddr + 16, r[1]);
+  for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(v[e]);
+  tc::tmem_st16(taddr, r);
 }
-// 32 values into slabs s0..s0+3 of a row-major tile, row t
-__device__ __forceinline__ void store_row32(uint8_t *tile, int t, int s0, const float (&v)[32]) {
+// 16 values into slabs s0, s0+1 of a row-major tile, row t
+__device__ __forceinline__ void store_row16(uint8_t *tile, int t, int s0, const float (&v)[16]) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < 2; ++c) {
     uint4 w;
     w.x = pack_bf16(v[8 * c + 0], v[8 * c + 1]);
     w.y = pack_bf16(v[8 * c + 2], v[8 * c + 3]);
@@ -305,20 +373,21 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
           *sW2T = smem + S::W2T;
   float *sB = reinterpret_cast<float *>(smem + S::BIAS);
   const float *sW3f = reinterpret_cast<const float *>(smem + S::W3F);
+  float4 *sW3r = reinterpret_cast<float4 *>(smem + S::W3R);
   float4 *sXch = reinterpret_cast<float4 *>(smem + S::XCH);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int t = ((warp & 3) << 5) | (tid & 31);  // tile row = Tensor Memory lane
-  const int hh = warp >> 2;                      // column half of the 64-wide layers
-  const int c0 = 32 * hh;
-  const int pair_bar = 1 + (warp & 3);  // named barrier of warps w and w + 4 (one row each)
+  const int hh = warp >> 2;                      // column group of the 64-wide layers
+  const int c0 = kCols * hh;
+  const int row_bar = 1 + (warp & 3);  // named barrier of the four warps of the same rows
 
-  load_weights(P, sW1, sW2, sW2T, sB, reinterpret_cast<float *>(smem + S::W3F));
+  dep_begin();
   if (tid < kRows) {
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      *reinterpret_cast<uint4 *>(sX[b] + 14 * kSlab + tid * 16) = make_uint4(0x3F80u, 0u, 0u, 0u);
-      *reinterpret_cast<uint4 *>(sX[b] + 15 * kSlab + tid * 16) = zero;
+      *reinterpret_cast<uint4 *>(sX[b] + 14 * kXPitch + tid * 16) = make_uint4(0x3F80u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4 *>(sX[b] + 15 * kXPitch + tid * 16) = zero;
     }
     *reinterpret_cast<uint4 *>(sDZ3 + kSlab + tid * 16) = zero;  // dz3 columns 8..15
   }
@@ -332,33 +401,33 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     tc::tmem_relinquish();
   }
 
-  // X rows of a tile: thread tid holds row tid % 128, slab pairs
-  // (tid / 128) + 2k (one aligned 32-byte sector of the row each)
-  uint4 xr[4][2];
+  // the parameters and gradients are the previous kernels' (an optimiser
+  // step, the gradient's reset)
+  dep_wait();
+  load_weights<kThreadsTrain>(P, sW1, sW2, sW2T, sB, reinterpret_cast<float *>(smem + S::W3F), sW3r);
+
+  // X rows of a tile: one run of 16-byte pieces, consecutive threads take
+  // consecutive ones (rows past n are zero)
+  constexpr int kPieces = kRows * kInSlabs, kIt = (kPieces + kThreadsTrain - 1) / kThreadsTrain;
+  uint4 xr[kIt];
   int ylab = -1, ycur = -1;  // labels of row tid (threads < 128)
   auto load_tile = [&](int64_t tile) {
-    const int64_t row = tile * kRows + (tid & (kRows - 1));
-    const bool valid = row < n;
-    const uint4 *src = reinterpret_cast<const uint4 *>(feat + (valid ? row : 0) * kIn);
+    const uint4 *src = reinterpret_cast<const uint4 *>(feat + tile * kRows * kIn);
+    const int64_t left = n - tile * kRows;
+    const int rows = (int)(left < kRows ? left : kRows);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int p = (tid >> 7) + 2 * k;
-      if (p < kIn / 16) {
-        xr[k][0] = valid ? __ldg(src + 2 * p) : make_uint4(0u, 0u, 0u, 0u);
-        xr[k][1] = valid ? __ldg(src + 2 * p + 1) : make_uint4(0u, 0u, 0u, 0u);
-      }
+    for (int k = 0; k < kIt; ++k) {
+      const int i = tid + k * kThreadsTrain;
+      xr[k] = i < rows * kInSlabs ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
     }
-    if (tid < kRows) ylab = valid ? (int)label[row] : -1;
+    if (tid < kRows) ylab = tid < rows ? (int)label[tile * kRows + tid] : -1;
   };
   auto store_tile = [&](uint8_t *dst) {
-    const int r = tid & (kRows - 1);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int p = (tid >> 7) + 2 * k;
-      if (p < kIn / 16) {
-        *reinterpret_cast<uint4 *>(dst + (2 * p) * kSlab + r * 16) = xr[k][0];
-        *reinterpret_cast<uint4 *>(dst + (2 * p + 1) * kSlab + r * 16) = xr[k][1];
-      }
+    for (int k = 0; k < kIt; ++k) {
+      const int i = tid + k * kThreadsTrain;
+      if (i < kPieces)
+        *reinterpret_cast<uint4 *>(dst + (i % kInSlabs) * kXPitch + (i / kInSlabs) * 16) = xr[k];
     }
   };
 
@@ -382,7 +451,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
   const float cw[3] = {cw0, cw1, cw2};
 
   if (tile < ntiles && tid == 0) {
-    mma_chain(tm, TT_D1, sX[0], kSlab, sW1, kHid * 16, kIn / 16, id64, false);
+    mma_chain(tm, TT_D1, sX[0], kXPitch, sW1, kWPitch, kIn / 16, id64, false);
     tc::mma_commit(&bar);
   }
   for (; tile < ntiles; tile += gridDim.x) {
@@ -391,18 +460,26 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     // ---- layer 1 done: h1, gelu'(z1)
     if (!(ok = wait_phase(&bar, phase, &abort_flag))) break;
     {
-      float v[32], gp[32];
-      tmem_row32(lane + TT_D1 + c0, v);
+      float v[kCols], gp[kCols];
+      tmem_row16(lane + TT_D1 + c0, v);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) gelu_and_grad(v[j] + sB[c0 + j], v[j], gp[j]);
-      store_row32(sH, t, 4 * hh, v);
-      tmem_store32(lane + TT_D1 + c0, gp);
+      for (int j = 0; j < kCols; j += 2) {
+        float2 g, d;
+        gelu_and_grad2(__fadd2_rn(make_float2(v[j], v[j + 1]),
+                                  *reinterpret_cast<const float2 *>(sB + c0 + j)), g, d);
+        v[j] = g.x;
+        v[j + 1] = g.y;
+        gp[j] = d.x;
+        gp[j + 1] = d.y;
+      }
+      store_row16(sH, t, 2 * hh, v);
+      tmem_store16(lane + TT_D1 + c0, gp);
       tc::tmem_wait_st();
     }
     tc::fence_async_smem();
     tc_sync();
     if (tid == 0) {
-      mma_chain(tm, TT_D2, sH, kSlab, sW2, kHid * 16, kHid / 16, id64, false);
+      mma_chain(tm, TT_D2, sH, kSlab, sW2, kWPitch, kHid / 16, id64, false);
       tc::mma_commit(&bar);
     }
     // ---- layer 2 done (and the previous tile's weight gradients): the
@@ -410,28 +487,46 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     if (!(ok = wait_phase(&bar, phase, &abort_flag))) break;
     if (has_next) load_tile(next);
     {
-      float h[32], gp[32];
-      tmem_row32(lane + TT_D2 + c0, h);
+      float h[kCols], gp[kCols];
+      tmem_row16(lane + TT_D2 + c0, h);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        gelu_and_grad(h[j] + sB[kHid + c0 + j], h[j], gp[j]);
-        h[j] = bf16_round(h[j]);  // the value the tile holds
+      for (int j = 0; j < kCols; j += 2) {
+        float2 g, d;
+        gelu_and_grad2(__fadd2_rn(make_float2(h[j], h[j + 1]),
+                                  *reinterpret_cast<const float2 *>(sB + kHid + c0 + j)), g, d);
+        h[j] = bf16_round(g.x);  // the values the tile holds
+        h[j + 1] = bf16_round(g.y);
+        gp[j] = d.x;
+        gp[j + 1] = d.y;
       }
-      store_row32(sH2, t, 4 * hh, h);
-      // logits: this half's partial sums, the other half's through smem
+      store_row16(sH2, t, 2 * hh, h);
+      // logits: this group's partial sums, the others' through smem
       float zp[3] = {0.0f, 0.0f, 0.0f};
+      {
+        float2 z01 = f2(0.0f);
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-#pragma unroll
-        for (int o = 0; o < kOut; ++o) zp[o] = fmaf(h[j], sW3f[o * kHid + c0 + j], zp[o]);
-      if (hh == 1) sXch[t] = make_float4(zp[0], zp[1], zp[2], 0.0f);
-      asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
+        for (int j = 0; j < kCols; ++j) {
+          const float4 w = sW3r[c0 + j];
+          z01 = __ffma2_rn(f2(h[j]), make_float2(w.x, w.y), z01);
+          zp[2] = fmaf(h[j], w.z, zp[2]);
+        }
+        zp[0] = z01.x;
+        zp[1] = z01.y;
+      }
+      if (hh > 0) sXch[hh * kRows + t] = make_float4(zp[0], zp[1], zp[2], 0.0f);
+      asm volatile("bar.sync %0, 128;" ::"r"(row_bar) : "memory");
       if (hh == 0) {
-        const float4 q = sXch[t];
+#pragma unroll
+        for (int k = 1; k < 4; ++k) {
+          const float4 q = sXch[k * kRows + t];
+          zp[0] += q.x;
+          zp[1] += q.y;
+          zp[2] += q.z;
+        }
         const int y = ycur;
         const float wy = (y >= 0 && y < kOut) ? cw[y] * inv_n : 0.0f;
-        const float z[3] = {zp[0] + q.x + sB[2 * kHid + 0], zp[1] + q.y + sB[2 * kHid + 1],
-                            zp[2] + q.z + sB[2 * kHid + 2]};
+        const float z[3] = {zp[0] + sB[2 * kHid + 0], zp[1] + sB[2 * kHid + 1],
+                            zp[2] + sB[2 * kHid + 2]};
         const float m = fmaxf(z[0], fmaxf(z[1], z[2]));
         float e[3], se = 0.0f;
 #pragma unroll
@@ -451,21 +546,24 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
             make_uint4(pack_bf16(dz[0], dz[1]), pack_bf16(dz[2], 0.0f), 0u, 0u);
         sXch[t] = make_float4(dz[0], dz[1], dz[2], 0.0f);
       }
-      asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
-      // dz2 = (dz3 W3) gelu'(z2) over this half's columns
+      asm volatile("bar.sync %0, 128;" ::"r"(row_bar) : "memory");
+      // dz2 = (dz3 W3) gelu'(z2) over this group's columns
       const float4 d3 = sXch[t];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float dh = fmaf(d3.x, sW3f[c0 + j],
-                              fmaf(d3.y, sW3f[kHid + c0 + j], d3.z * sW3f[2 * kHid + c0 + j]));
-        gp[j] *= dh;
+      for (int j = 0; j < kCols; j += 2) {
+        const float2 w0 = *reinterpret_cast<const float2 *>(sW3f + c0 + j),
+                     w1 = *reinterpret_cast<const float2 *>(sW3f + kHid + c0 + j),
+                     w2 = *reinterpret_cast<const float2 *>(sW3f + 2 * kHid + c0 + j);
+        const float2 dh = __ffma2_rn(f2(d3.x), w0, __ffma2_rn(f2(d3.y), w1, __fmul2_rn(f2(d3.z), w2)));
+        gp[j] *= dh.x;
+        gp[j + 1] *= dh.y;
       }
-      store_row32(sDZ2, t, 4 * hh, gp);
+      store_row16(sDZ2, t, 2 * hh, gp);
     }
     tc::fence_async_smem();
     tc_sync();
     if (tid == 0) {
-      mma_chain(tm, TT_D2, sDZ2, kSlab, sW2T, kHid * 16, kHid / 16, id64, false);
+      mma_chain(tm, TT_D2, sDZ2, kSlab, sW2T, kWPitch, kHid / 16, id64, false);
       tc::mma_commit(&bar);
       // [dW2 | dW3]^T += [h1 | h2]^T [dz2 | dz3] (K = the tile's rows)
       for (int s = 0; s < kRows / 16; ++s)
@@ -475,12 +573,12 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     // ---- dz1 = dh1 gelu'(z1); the next tile's rows into the other buffer
     if (!(ok = wait_phase(&bar, phase, &abort_flag))) break;
     {
-      float dh[32], gp[32];
-      tmem_row32(lane + TT_D2 + c0, dh);
-      tmem_row32(lane + TT_D1 + c0, gp);
+      float dh[kCols], gp[kCols];
+      tmem_row16(lane + TT_D2 + c0, dh);
+      tmem_row16(lane + TT_D1 + c0, gp);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) dh[j] *= gp[j];
-      store_row32(sDZ, t, 4 * hh, dh);
+      for (int j = 0; j < kCols; ++j) dh[j] *= gp[j];
+      store_row16(sDZ, t, 2 * hh, dh);
     }
     if (has_next) store_tile(sX[b ^ 1]);
     ycur = ylab;
@@ -488,12 +586,12 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     tc_sync();
     if (tid == 0) {
       if (has_next) {
-        mma_chain(tm, TT_D1, sX[b ^ 1], kSlab, sW1, kHid * 16, kIn / 16, id64, false);
+        mma_chain(tm, TT_D1, sX[b ^ 1], kXPitch, sW1, kWPitch, kIn / 16, id64, false);
         tc::mma_commit(&bar);
       }
       // [dW1 | db1 db2 db3]^T += [x | 1]^T [dz1 | dz2 | dz3]
       for (int s = 0; s < kRows / 16; ++s)
-        tc::mma_bf16(tm + TT_G1, tc::smem_desc(sX[b] + 256 * s, 128, kSlab),
+        tc::mma_bf16(tm + TT_G1, tc::smem_desc(sX[b] + 256 * s, 128, kXPitch),
                      tc::smem_desc(sDZ + 256 * s, 128, kSlab), id_g1, (any || s > 0) ? 1u : 0u);
       if (!has_next) tc::mma_commit(&bar);
     }
@@ -505,9 +603,9 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
   if (ok && any) {
     // lanes of [h1|h2]^T [dz2|dz3]: hidden unit t of h1 (t < 64) or h2
     if (t < kHid) {
-      float c[32];
-      tmem_row32(lane + TT_GCAT + c0, c);
-      for (int o = 0; o < 32; ++o) atomicAdd(&grad[P_W2 + (c0 + o) * kHid + t], c[o]);
+      float c[kCols];
+      tmem_row16(lane + TT_GCAT + c0, c);
+      for (int o = 0; o < kCols; ++o) atomicAdd(&grad[P_W2 + (c0 + o) * kHid + t], c[o]);
     } else if (hh == 0) {
       uint32_t r[16];
       tc::tmem_ld16(lane + TT_GCAT + kHid, r);
@@ -516,20 +614,20 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
     }
     // lanes of [x|1]^T [dz1|dz2|dz3]: input feature t, or the ones row
     {
-      float c[32];
-      tmem_row32(lane + TT_G1 + c0, c);
+      float c[kCols];
+      tmem_row16(lane + TT_G1 + c0, c);
       if (t < kIn) {
-        for (int o = 0; o < 32; ++o) atomicAdd(&grad[P_W1 + (c0 + o) * kIn + t], c[o]);
+        for (int o = 0; o < kCols; ++o) atomicAdd(&grad[P_W1 + (c0 + o) * kIn + t], c[o]);
       } else if (t == kOnesRow) {
-        for (int o = 0; o < 32; ++o) atomicAdd(&grad[P_B1 + c0 + o], c[o]);
+        for (int o = 0; o < kCols; ++o) atomicAdd(&grad[P_B1 + c0 + o], c[o]);
       }
     }
     if ((warp & 3) == (kOnesRow >> 5)) {
       // the ones row's dz2 and dz3 columns: db2 and db3
-      float c[32];
-      tmem_row32(lane + TT_G1 + kHid + c0, c);
+      float c[kCols];
+      tmem_row16(lane + TT_G1 + kHid + c0, c);
       if (t == kOnesRow)
-        for (int o = 0; o < 32; ++o) atomicAdd(&grad[P_B2 + c0 + o], c[o]);
+        for (int o = 0; o < kCols; ++o) atomicAdd(&grad[P_B2 + c0 + o], c[o]);
       if (hh == 0) {
         uint32_t r[16];
         tc::tmem_ld16(lane + TT_G1 + 2 * kHid, r);
@@ -564,23 +662,62 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
 // Layer 2's activations and the logits of this thread's row (one thread per
 // row): h2 = gelu(z2 + b2) rounded to bf16, z3 = h2 W3^T + b3 accumulated
 // in f32 on the CUDA cores (W3 has 3 rows: no third MMA round trip).
-__device__ __forceinline__ void logits_row(uint32_t taddr_d2, const float *sB, const float *sW3f,
+__device__ __forceinline__ void logits_row(uint32_t taddr_d2, const float *sB, const float4 *sW3r,
                                            float (&z)[3]) {
-  float h[64];
-  tmem_row64(taddr_d2, sB + kHid, h);
+  float2 z01 = make_float2(sB[2 * kHid], sB[2 * kHid + 1]);
+  float z2 = sB[2 * kHid + 2];
 #pragma unroll
-  for (int o = 0; o < kOut; ++o) z[o] = sB[2 * kHid + o];
+  for (int c = 0; c < kHid; c += 32) {
+    float h[32];
+    tmem_row32(taddr_d2 + c, h);
 #pragma unroll
-  for (int j = 0; j < kHid; ++j) {
-    const float g = bf16_round(gelu(h[j]));
+    for (int j = 0; j < 32; j += 2) {
+      const float2 g = gelu2(__fadd2_rn(make_float2(h[j], h[j + 1]),
+                                        *reinterpret_cast<const float2 *>(sB + kHid + c + j)));
+      const float a = bf16_round(g.x), b = bf16_round(g.y);
+      const float4 wa = sW3r[c + j], wb = sW3r[c + j + 1];
+      z01 = __ffma2_rn(f2(a), make_float2(wa.x, wa.y), z01);
+      z2 = fmaf(a, wa.z, z2);
+      z01 = __ffma2_rn(f2(b), make_float2(wb.x, wb.y), z01);
+      z2 = fmaf(b, wb.z, z2);
+    }
+  }
+  z[0] = z01.x;
+  z[1] = z01.y;
+  z[2] = z2;
+}
+
+// Layer 1's activations of this thread's row, 32 columns at a time, into the
+// h1 tile.
+template <int PITCH>
+__device__ __forceinline__ void hidden_row(uint32_t taddr_d1, const float *sB, uint8_t *tile,
+                                           int t) {
 #pragma unroll
-    for (int o = 0; o < kOut; ++o) z[o] = fmaf(g, sW3f[o * kHid + j], z[o]);
+  for (int c = 0; c < kHid; c += 32) {
+    float v[32];
+    tmem_row32(taddr_d1 + c, v);
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = j + 2 * k;
+        const float2 g = gelu2(__fadd2_rn(make_float2(v[e], v[e + 1]),
+                                          *reinterpret_cast<const float2 *>(sB + c + e)));
+        w[k] = pack_bf16(g.x, g.y);
+      }
+      *reinterpret_cast<uint4 *>(tile + ((c + j) / 8) * PITCH + t * 16) =
+          make_uint4(w[0], w[1], w[2], w[3]);
+    }
   }
 }
 
 // ---------------------------------------------------------------------------
-// Inference: logits and argmax class per row.
-__global__ void __launch_bounds__(kThreads)
+// Inference: logits and argmax class per row.  Bound by memory latency and
+// issue together (32 % of the slots, four CTAs per SM): 200,003 rows 60 -> 31
+// us; the uncoalesced tile loads and the weights loaded one by one had cost
+// the rest, at any occupancy.
+__global__ void __launch_bounds__(kThreads, kFwdCtas)
     mlp_forward_kernel(const float *__restrict__ P, const uint16_t *__restrict__ feat, int64_t n,
                        uint8_t *__restrict__ cls, float *__restrict__ logits, int *__restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -590,9 +727,9 @@ __global__ void __launch_bounds__(kThreads)
   using S = FwdSmem;
   uint8_t *sX = smem + S::X, *sH1 = smem + S::H1, *sW1 = smem + S::W1, *sW2 = smem + S::W2;
   float *sB = reinterpret_cast<float *>(smem + S::BIAS);
-  float *sW3f = reinterpret_cast<float *>(smem + S::W3F);
+  float4 *sW3r = reinterpret_cast<float4 *>(smem + S::W3R);
   const int t = threadIdx.x;
-  load_weights(P, sW1, sW2, nullptr, sB, sW3f);
+  load_weights<kThreads>(P, sW1, sW2, nullptr, sB, nullptr, sW3r);
   if (t == 0) {
     tc::mbar_init(&bar, 1);
     abort_flag = 0;
@@ -612,25 +749,19 @@ __global__ void __launch_bounds__(kThreads)
   for (int64_t tile = blockIdx.x; ok && tile * kRows < n; tile += gridDim.x) {
     const int64_t row = tile * kRows + t;
     const bool valid = row < n;
-    load_x_row(feat, row, valid, t, sX);
+    load_x_tile(feat, tile, n, t, sX);
     tc::fence_async_smem();
     tc_sync();
-    if (t == 0) mma_chain(tm, T_D1, sX, kRows * 16, sW1, kHid * 16, kIn / 16, id64, false);
+    if (t == 0) mma_chain(tm, T_D1, sX, kXPitch, sW1, kWPitch, kIn / 16, id64, false);
     if (!(ok = commit_and_wait(&bar, phase, &abort_flag))) break;
-    {
-      float v[64];
-      tmem_row64(tm + lane_off + T_D1, sB, v);
-#pragma unroll
-      for (int j = 0; j < kHid; ++j) v[j] = gelu(v[j]);
-      store_row64(sH1, t, v);
-    }
+    hidden_row<kXPitch>(tm + lane_off + T_D1, sB, sH1, t);
     tc::fence_async_smem();
     tc_sync();
-    if (t == 0) mma_chain(tm, T_D2, sH1, kRows * 16, sW2, kHid * 16, kHid / 16, id64, false);
+    if (t == 0) mma_chain(tm, T_D2, sH1, kXPitch, sW2, kWPitch, kHid / 16, id64, false);
     if (!(ok = commit_and_wait(&bar, phase, &abort_flag))) break;
     {
       float z[3];
-      logits_row(tm + lane_off + T_D2, sB, sW3f, z);
+      logits_row(tm + lane_off + T_D2, sB, sW3r, z);
       int am = 0;
       if (z[1] > z[am]) am = 1;
       if (z[2] > z[am]) am = 2;
@@ -654,9 +785,18 @@ __global__ void __launch_bounds__(kThreads)
   if ((t >> 5) == 0) tc::tmem_dealloc(tm, T_COLS_FWD);
 }
 
+// the gradient's reset before a training step's gradient kernel
+__global__ void zero_kernel(float *__restrict__ g, int n) {
+  dep_begin();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) g[i] = 0.0f;
+}
+
 __global__ void adam_kernel(float *__restrict__ P, const float *__restrict__ g, float *__restrict__ m,
                             float *__restrict__ v, int n, float lr, float c1, float c2) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  dep_begin();
+  dep_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -781,15 +921,15 @@ __global__ void features_kernel(FeatConst F, int64_t n, const int64_t *__restric
 // memory: X, h1, weights; Tensor Memory: 128 columns (D1 0..63, D2
 // 64..127) so several CTAs share an SM.
 struct MeshSmem {
+  static constexpr int kPitch = kRows * 16;  // rows are stored by their own thread: no padding
   static constexpr int X = 0;
-  static constexpr int H1 = X + kRows * kIn * 2;
-  static constexpr int W1 = H1 + kRows * kHid * 2;
-  static constexpr int W2 = W1 + kHid * kIn * 2;
-  static constexpr int BIAS = W2 + kHid * kHid * 2;
-  static constexpr int W3F = BIAS + 1024;  // W3 rounded to bf16, as f32 [3 x 64]
-  static constexpr int BYTES = W3F + 1024;
+  static constexpr int H1 = X;
+  static constexpr int W1 = X + kInSlabs * kPitch;
+  static constexpr int W2 = W1 + kInSlabs * kWPitch;
+  static constexpr int BIAS = W2 + kHid / 8 * kWPitch;
+  static constexpr int W3R = BIAS + 544;  // W3 rounded to bf16, as f32 [64 x 4]
+  static constexpr int BYTES = W3R + 1024;
 };
-constexpr uint32_t T_COLS_MESH = 128;
 
 struct MeshArgs {
   const int32_t *tile_nb, *tile_level;
@@ -834,7 +974,7 @@ __global__ void class_to_tag_kernel(const uint8_t *__restrict__ cls, int64_t n,
     out[i] = masked_tag(cls[i], lvl[i], refine, coarsen);
 }
 
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, kFwdCtas)
     mlp_tag_mesh_kernel(const float *__restrict__ P, MeshArgs m, FeatScale F, int *__restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t bar;
@@ -846,16 +986,16 @@ __global__ void __launch_bounds__(kThreads)
   using S = MeshSmem;
   uint8_t *sX = smem + S::X, *sH1 = smem + S::H1, *sW1 = smem + S::W1, *sW2 = smem + S::W2;
   float *sB = reinterpret_cast<float *>(smem + S::BIAS);
-  float *sW3f = reinterpret_cast<float *>(smem + S::W3F);
+  float4 *sW3r = reinterpret_cast<float4 *>(smem + S::W3R);
   const int t = threadIdx.x;
-  load_weights(P, sW1, sW2, nullptr, sB, sW3f);
+  load_weights<kThreads>(P, sW1, sW2, nullptr, sB, nullptr, sW3r);
   if (t == 0) {
     tc::mbar_init(&bar, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if ((t >> 5) == 0) {
-    tc::tmem_alloc(&tbase, T_COLS_MESH);
+    tc::tmem_alloc(&tbase, T_COLS_FWD);
     tc::tmem_relinquish();
   }
   tc::fence_async_smem();
@@ -938,27 +1078,21 @@ __global__ void __launch_bounds__(kThreads)
         w.y = pack_bf16(fv[8 * c + 2], fv[8 * c + 3]);
         w.z = pack_bf16(fv[8 * c + 4], fv[8 * c + 5]);
         w.w = pack_bf16(fv[8 * c + 6], fv[8 * c + 7]);
-        *reinterpret_cast<uint4 *>(sX + c * (kRows * 16) + t * 16) = w;
+        *reinterpret_cast<uint4 *>(sX + c * S::kPitch + t * 16) = w;
       }
     }
     tc::fence_async_smem();
     tc_sync();
-    if (t == 0) mma_chain(tm, 0, sX, kRows * 16, sW1, kHid * 16, kIn / 16, id64, false);
+    if (t == 0) mma_chain(tm, T_D1, sX, S::kPitch, sW1, kWPitch, kIn / 16, id64, false);
     if (!(ok = commit_and_wait(&bar, phase, &abort_flag))) break;
-    {
-      float h[64];
-      tmem_row64(tm + lane_off + 0, sB, h);
-#pragma unroll
-      for (int j = 0; j < kHid; ++j) h[j] = gelu(h[j]);
-      store_row64(sH1, t, h);
-    }
+    hidden_row<S::kPitch>(tm + lane_off + T_D1, sB, sH1, t);
     tc::fence_async_smem();
     tc_sync();
-    if (t == 0) mma_chain(tm, 64, sH1, kRows * 16, sW2, kHid * 16, kHid / 16, id64, false);
+    if (t == 0) mma_chain(tm, T_D2, sH1, S::kPitch, sW2, kWPitch, kHid / 16, id64, false);
     if (!(ok = commit_and_wait(&bar, phase, &abort_flag))) break;
     {
       float z[3];
-      logits_row(tm + lane_off + 64, sB, sW3f, z);
+      logits_row(tm + lane_off + T_D2, sB, sW3r, z);
       int am = 0;
       if (z[1] > z[am]) am = 1;
       if (z[2] > z[am]) am = 2;
@@ -974,7 +1108,7 @@ __global__ void __launch_bounds__(kThreads)
     tc::mbar_wait_bounded(&bar, phase, kWaitCycles);
   }
   tc_sync();
-  if ((t >> 5) == 0) tc::tmem_dealloc(tm, T_COLS_MESH);
+  if ((t >> 5) == 0) tc::tmem_dealloc(tm, T_COLS_FWD);
 }
 
 // Plain criterion over every normal cell of the context (centres from the
@@ -1154,22 +1288,22 @@ int features_impl(const CtxView &V, const ibgpu_ctx *ctx, const ibgpu_tag_rule *
 
 int launch_grad(const CtxView &V, const float *d_params, int64_t n, const uint16_t *d_feat,
                 const uint8_t *d_label, const float class_weight[3], float *d_grad,
-                float *d_stats) {
+                float *d_stats, bool dep) {
   const int64_t tiles = (n + kRows - 1) / kRows;
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)V.nsm);
-  mlp_grad_kernel<<<grid, kThreadsTrain, TrainSmem::BYTES, V.stream>>>(
-      d_params, d_feat, d_label, n, class_weight[0], class_weight[1], class_weight[2],
-      (float)(1.0 / (double)n), d_grad, d_stats, V.aux_err);
+  launch_dep_smem(dep, V.stream, grid, kThreadsTrain, TrainSmem::BYTES, mlp_grad_kernel, d_params,
+                  d_feat, d_label, n, class_weight[0], class_weight[1], class_weight[2],
+                  (float)(1.0 / (double)n), d_grad, d_stats, V.aux_err);
   CKI(cudaGetLastError());
   return IBGPU_OK;
 }
 
 int launch_adam(const CtxView &V, float *d_params, const float *d_grad, float *d_m, float *d_v,
-                int step, float lr) {
+                int step, float lr, bool dep) {
   const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, step)));
   const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, step)));
-  adam_kernel<<<grid_for(P_COUNT, V.nsm, 256), 256, 0, V.stream>>>(d_params, d_grad, d_m, d_v,
-                                                                   P_COUNT, lr, c1, c2);
+  launch_dep(dep, V.stream, grid_for(P_COUNT, V.nsm, 256), 256, adam_kernel, d_params, d_grad, d_m,
+             d_v, P_COUNT, lr, c1, c2);
   CKI(cudaGetLastError());
   return IBGPU_OK;
 }
@@ -1179,7 +1313,7 @@ int forward_impl(const CtxView &V, const float *d_params, int64_t n, const uint1
   int rc = configure_smem();
   if (rc) return rc;
   const int64_t tiles = (n + kRows - 1) / kRows;
-  const int grid = (int)std::min<int64_t>(tiles, (int64_t)V.nsm * 2);
+  const int grid = (int)std::min<int64_t>(tiles, (int64_t)V.nsm * kFwdCtas);
   mlp_forward_kernel<<<grid, kThreads, FwdSmem::BYTES, V.stream>>>(d_params, d_feat, n, d_class,
                                                                    d_logits, V.aux_err);
   CKI(cudaGetLastError());
@@ -1227,7 +1361,7 @@ int tag_mesh_enqueue(ibgpu_ctx *ctx, const ibgpu_tag_rule *rule, const float *d_
   request_masks(rule, F.refine_levels, F.coarsen_levels);
   if (d_params) {
     const int64_t items = V.nslots / kRows;
-    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)V.nsm * 3));
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)V.nsm * kFwdCtas));
     mlp_tag_mesh_kernel<<<grid, kThreads, MeshSmem::BYTES, st>>>(d_params, m, F, V.aux_err);
   } else {
     tag_plain_mesh_kernel<<<grid_for(V.nslots, V.nsm, 256), 256, 0, st>>>(to_dev(rule), m, F);
@@ -1299,7 +1433,7 @@ int ibgpu_mlp_grad(ibgpu_ctx *ctx, const float *d_params, int64_t n, const uint1
   if ((reinterpret_cast<uintptr_t>(d_feat) & 15u) != 0) return IBGPU_E_ARG;
   int rc = configure_smem();
   if (rc) return rc;
-  rc = launch_grad(V, d_params, n, d_feat, d_label, class_weight, d_grad, d_stats);
+  rc = launch_grad(V, d_params, n, d_feat, d_label, class_weight, d_grad, d_stats, false);
   if (rc) return rc;
   return kernel_error_check(V.aux_err, V.stream);
 }
@@ -1314,10 +1448,11 @@ int ibgpu_mlp_train_step(ibgpu_ctx *ctx, float *d_params, float *d_m, float *d_v
   if ((reinterpret_cast<uintptr_t>(d_feat) & 15u) != 0) return IBGPU_E_ARG;
   int rc = configure_smem();
   if (rc) return rc;
-  CKI(cudaMemsetAsync(d_grad, 0, (size_t)P_COUNT * sizeof(float), V.stream));
-  rc = launch_grad(V, d_params, n, d_feat, d_label, class_weight, d_grad, d_stats);
+  launch_dep(false, V.stream, (P_COUNT + 255) / 256, 256, zero_kernel, d_grad, P_COUNT);
+  CKI(cudaGetLastError());
+  rc = launch_grad(V, d_params, n, d_feat, d_label, class_weight, d_grad, d_stats, true);
   if (rc) return rc;
-  rc = launch_adam(V, d_params, d_grad, d_m, d_v, step, lr);
+  rc = launch_adam(V, d_params, d_grad, d_m, d_v, step, lr, true);
   if (rc) return rc;
   return kernel_error_check(V.aux_err, V.stream);
 }
@@ -1327,7 +1462,7 @@ int ibgpu_mlp_adam(ibgpu_ctx *ctx, float *d_params, const float *d_grad, float *
   CtxView V;
   if (ctx_view(ctx, &V) != IBGPU_OK || step < 1 || !d_params || !d_grad || !d_m || !d_v)
     return IBGPU_E_ARG;
-  return launch_adam(V, d_params, d_grad, d_m, d_v, step, lr);
+  return launch_adam(V, d_params, d_grad, d_m, d_v, step, lr, false);
 }
 
 int ibgpu_tag_learned(ibgpu_ctx *ctx, const ibgpu_tag_rule *rule, const ibgpu_tag_cells *cells,

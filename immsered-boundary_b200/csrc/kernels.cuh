@@ -13,6 +13,7 @@
 #include <mutex>
 #include <stdint.h>
 
+#include "dependent.cuh"
 #include "flux.cuh"
 #include "layout.h"
 
@@ -23,32 +24,6 @@ constexpr int kHalo = 2;
 constexpr int kReg = kTile + 2 * kHalo;  // 20: tile plus a 2-cell halo
 constexpr int kXFaces = kTile * (kTile + 1);
 constexpr int kYFaces = (kTile + 1) * kTile;
-
-// Programmatic dependent launch: a kernel of the step lets the next one be
-// set up as soon as all its CTAs run, and waits for the previous one to have
-// completed before it reads or writes anything that the step changes (mesh
-// tables, which no kernel of a run writes, may be read before).
-__device__ __forceinline__ void dep_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void dep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... P, typename... A>
-void launch_dep(bool dep, cudaStream_t st, dim3 grid, dim3 block, void (*kernel)(P...),
-                const A &...args) {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = dep ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
 
 // What a step's first stage resets (StageArgs::reset); nothing reads these
 // words before the step's final stage.
