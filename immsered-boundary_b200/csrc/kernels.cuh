@@ -13,6 +13,7 @@
 #include <mutex>
 #include <stdint.h>
 
+#include "cfl.cuh"
 #include "dependent.cuh"
 #include "flux.cuh"
 #include "layout.h"
@@ -33,30 +34,6 @@ __device__ __forceinline__ void step_reset(const StageArgs &a) {
       for (int c = 0; c < 5; ++c) a.diag->res_bits[c] = 0ull;
     if (a.reset & 2) a.diag->cfl_bits = (unsigned long long)__double_as_longlong(10000.0);
   }
-}
-
-__device__ __forceinline__ void raise_error(DevDiag *d, int phase, int check, int slot) {
-  unsigned long long key = ((unsigned long long)phase << 40) |
-                           ((unsigned long long)check << 32) | (unsigned)slot;
-  atomicMin(&d->err_key, key);
-}
-
-// Exact maximum / minimum of a 64-bit word over the full warp with the
-// 32-bit warp reductions (redux.sync): the extreme high word first, then the
-// extreme low word among the lanes that hold it.  Four instructions instead
-// of five rounds of two 32-bit shuffles and a 64-bit compare.
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return ((unsigned long long)mh << 32) | ml;
-}
-
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
-  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
-  const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? lo : 0xffffffffu);
-  return ((unsigned long long)mh << 32) | ml;
 }
 
 // Threads of a fast-build stage CTA: FP64 adds a ninth warp that owns the
@@ -108,23 +85,6 @@ __device__ __forceinline__ void block_resnorm(const unsigned long long (&rb)[4],
     unsigned long long *dst = &d->res_bits[tid == 3 ? 4 : tid];
     atomicMax(dst, m);  // result unused: a reduction the CTA does not wait for
   }
-}
-
-// CFL bound of one normal cell, NS_Solver::Comptdt (NS_Solver.cpp:196-280),
-// with every operation separately rounded so the CFL pass and the final
-// stages that fold it in produce the same bits in every build: cfl_vol over
-// the sum of the cell's wave speeds times face areas.
-__device__ __forceinline__ double cfl_cell_sum(double T, double u, double v, const LevelConst &L,
-                                               const CaseConst &cc) {
-  const double c = __dsqrt_rn(__dmul_rn(cc.gamaRg, T));
-  const double c0 = __dmul_rn(__dadd_rn(fabs(u), c), L.area_x);
-  const double c1 = __dmul_rn(__dadd_rn(fabs(v), c), L.area_y);
-  const double c2 = __dmul_rn(__dadd_rn(0.0, c), L.area_z);
-  return __dadd_rn(__dadd_rn(c0, c1), c2);
-}
-__device__ __forceinline__ double cfl_cell_bound(double T, double u, double v, const LevelConst &L,
-                                                 const CaseConst &cc) {
-  return __ddiv_rn(L.cfl_vol, cfl_cell_sum(T, u, v, L, cc));
 }
 
 // The next step's CFL pass folded into a final stage: the sum of each

@@ -508,8 +508,8 @@ void ibgpu_batch_destroy(ibgpu_batch *b);
  * cudaMalloc, cudaFree or allocating library routine is called.  nx and ny
  * must be multiples of 16 with nx * ny <= IBGPU_NOALLOC_MAX_CELLS, else
  * IBGPU_E_ARG.  The first call on a device looks up that array's address
- * (once per device, with the device current): make it before any stream
- * capture.  All calls share the array, which keeps the last call's contents;
+ * and registers one static host page that returns dt and diag (once per
+ * device, with the device current): make it before any stream capture.  All calls share the array, which keeps the last call's contents;
  * calls that overlap on the GPU race, so the caller serialises them.  The
  * call synchronises `stream` (a cudaStream_t, NULL for the legacy stream)
  * to return dt and diag. */
