@@ -21,10 +21,16 @@ struct CtxView {
   const int2 *tile_org;
   const int32_t *cell_slot;
   int64_t ncells, nslots, ntiles;
-  int *aux_err;  // device word: set by a kernel whose wait ran out of time
+  int *aux_err, *aux_err_host;  // set by a kernel whose wait ran out of time (mapped)
   CaseConst cc;
 };
 int ctx_view(const ibgpu_ctx *ctx, CtxView *v);
+// Whether the (synchronised) kernels of a context timed out; clears the word.
+inline bool aux_timed_out(volatile int *word) {
+  const bool t = *word != 0;
+  if (t) *word = 0;
+  return t;
+}
 // per-slot signed wall distance (created on demand); tag buffer of nslots
 // per-slot bytes followed by ncells per-row bytes
 int ctx_signdis_buffer(ibgpu_ctx *ctx, double **dev, bool create);

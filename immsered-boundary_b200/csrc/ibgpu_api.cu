@@ -119,7 +119,9 @@ struct ibgpu_ctx {
   double *d_rows = nullptr;  // staging for AoS state transfers
   DevDiag *d_diag = nullptr;
   DevDiag *h_diag = nullptr;  // pinned
-  int *d_aux_err = nullptr;   // time-out flag of the indicator kernels
+  // time-out flag of the indicator kernels, in mapped host memory: read after
+  // the stream's synchronisation without a copy (15 us a call from pageable)
+  int *h_aux_err = nullptr, *d_aux_err = nullptr;
 
   // slot lookup: per level, tile (tx,ty) -> tile index
   std::vector<std::unordered_map<uint64_t, int>> tilemap;
@@ -359,6 +361,7 @@ int ctx_view(const ibgpu_ctx *ctx, CtxView *v) {
   v->nslots = ctx->nslots;
   v->ntiles = ctx->ntiles;
   v->aux_err = ctx->d_aux_err;
+  v->aux_err_host = ctx->h_aux_err;
   v->cc = ctx->cc;
   return IBGPU_OK;
 }
@@ -528,9 +531,13 @@ int ibgpu_create(const ibgpu_case *cs, ibgpu_ctx **out) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_in_free, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_in_done, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_diag, sizeof(DevDiag));
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_diag, sizeof(DevDiag));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_aux_err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->d_aux_err, 0, sizeof(int));
+  // one pinned (and mapped) allocation: the diagnostics, then the flag
+  if (e == cudaSuccess) e = cudaHostAlloc((void **)&c->h_diag, sizeof(DevDiag) + 64, cudaHostAllocMapped);
+  if (e == cudaSuccess) {
+    c->h_aux_err = reinterpret_cast<int *>(c->h_diag + 1);
+    *c->h_aux_err = 0;
+    e = cudaHostGetDevicePointer((void **)&c->d_aux_err, c->h_aux_err, 0);
+  }
   if (e != cudaSuccess) {
     int rc = cuda_fail(e, "ibgpu_create");
     ibgpu_destroy(c);
@@ -1510,7 +1517,6 @@ struct ibgpu_batch {
   int table = -1;       // byte offset of the arguments in the constant-memory table (-1: global)
   int table_bytes = 0;  // bytes reserved there
   bool tuned = false;
-  int *h_err = nullptr;  // pinned: the cases' time-out flags (batch tagging)
   std::vector<cudaEvent_t> ev_tag;  // batch tagging: per case, + the fork
   int fixed_grid = -1;  // >= 0: CTA count set by the caller (no autotuning)
   int threads = 0;        // threads per CTA of the merged stage launch (256 / 288)
@@ -1555,8 +1561,6 @@ struct ibgpu_batch {
     fast::batch_table_release(device, table);
     table = -1;
     table_bytes = 0;
-    if (h_err) cudaFreeHost(h_err);
-    h_err = nullptr;
     for (auto e : ev_tag) cudaEventDestroy(e);
     ev_tag.clear();
   }
@@ -2130,8 +2134,7 @@ int ibgpu_batch_tag_mesh(ibgpu_batch *b, const ibgpu_tag_rule *rule, const float
   // each case tags on its own stream after the batch's pending work (the
   // cases' kernels overlap, so one case's last partial wave does not idle the
   // GPU), its rows copied back behind its kernels; the batch stream then
-  // waits for all of them and reads every time-out flag in one
-  // synchronisation
+  // waits for all of them: one synchronisation
   const size_t n = b->cases.size();
   if (b->ev_tag.size() != n + 1) {
     for (auto e : b->ev_tag) cudaEventDestroy(e);
@@ -2152,21 +2155,11 @@ int ibgpu_batch_tag_mesh(ibgpu_batch *b, const ibgpu_tag_rule *rule, const float
     CK(cudaStreamWaitEvent(st, b->ev_tag[i], 0));
     off += c->ncells;
   }
-  if (d_params) {
-    if (!b->h_err) CK(cudaHostAlloc((void **)&b->h_err, n * sizeof(int), cudaHostAllocDefault));
-    for (size_t i = 0; i < n; ++i)
-      CK(cudaMemcpyAsync(b->h_err + i, b->cases[i]->d_aux_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  }
   CK(cudaStreamSynchronize(st));
   if (d_params) {
     bool timed_out = false;
-    for (size_t i = 0; i < n; ++i)
-      if (b->h_err[i]) {
-        timed_out = true;
-        CK(cudaMemsetAsync(b->cases[i]->d_aux_err, 0, sizeof(int), st));
-      }
+    for (ibgpu_ctx *c : b->cases) timed_out = aux_timed_out(c->h_aux_err) || timed_out;
     if (timed_out) {
-      CK(cudaStreamSynchronize(st));
       g_last_error = "tensor-core wait ran out of its time limit";
       return IBGPU_E_TIMEOUT;
     }
@@ -2539,7 +2532,6 @@ void ibgpu_destroy(ibgpu_ctx *ctx) {
   ctx->free_layout();
   ibgpu::wall_free(ctx->wall);
   cudaFree(ctx->d_diag);
-  cudaFree(ctx->d_aux_err);
   cudaFreeHost(ctx->h_diag);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->in_stream) cudaStreamDestroy(ctx->in_stream);

@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1)
   }
   if (!ok) {
     if (tid == 0) {
-      atomicExch(err, 1);
+      *static_cast<volatile int *>(err) = 1;
       tc::mma_commit(&bar);
     }
     // let the MMAs already issued finish (bounded) before freeing their memory
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kThreads, kFwdCtas)
     // loads above (tc_sync at the top of the loop)
   }
   if (!ok) {
-    if (t == 0) atomicExch(err, 1);
+    if (t == 0) *static_cast<volatile int *>(err) = 1;
     tc::mbar_wait_bounded(&bar, phase, kWaitCycles);
   }
   tc_sync();
@@ -1104,7 +1104,7 @@ __global__ void __launch_bounds__(kThreads, kFwdCtas)
     // follows its staging (every lane read above by then)
   }
   if (!ok) {
-    if (t == 0) atomicExch(err, 1);
+    if (t == 0) *static_cast<volatile int *>(err) = 1;
     tc::mbar_wait_bounded(&bar, phase, kWaitCycles);
   }
   tc_sync();
@@ -1224,13 +1224,9 @@ int upload(DevBuf &b, const T *h, int64_t n, cudaStream_t st) {
   return IBGPU_OK;
 }
 
-int kernel_error_check(int *d_err, cudaStream_t st) {
-  int h = 0;
-  CKI(cudaMemcpyAsync(&h, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CKI(cudaStreamSynchronize(st));
-  if (h) {
-    CKI(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-    CKI(cudaStreamSynchronize(st));
+int kernel_error_check(const CtxView &V) {
+  CKI(cudaStreamSynchronize(V.stream));
+  if (aux_timed_out(V.aux_err_host)) {
     set_last_error("tensor-core wait ran out of its time limit");
     return IBGPU_E_TIMEOUT;
   }
@@ -1317,7 +1313,7 @@ int forward_impl(const CtxView &V, const float *d_params, int64_t n, const uint1
   mlp_forward_kernel<<<grid, kThreads, FwdSmem::BYTES, V.stream>>>(d_params, d_feat, n, d_class,
                                                                    d_logits, V.aux_err);
   CKI(cudaGetLastError());
-  return kernel_error_check(V.aux_err, V.stream);
+  return kernel_error_check(V);
 }
 
 }  // namespace
@@ -1435,7 +1431,7 @@ int ibgpu_mlp_grad(ibgpu_ctx *ctx, const float *d_params, int64_t n, const uint1
   if (rc) return rc;
   rc = launch_grad(V, d_params, n, d_feat, d_label, class_weight, d_grad, d_stats, false);
   if (rc) return rc;
-  return kernel_error_check(V.aux_err, V.stream);
+  return kernel_error_check(V);
 }
 
 int ibgpu_mlp_train_step(ibgpu_ctx *ctx, float *d_params, float *d_m, float *d_v, float *d_grad,
@@ -1454,7 +1450,7 @@ int ibgpu_mlp_train_step(ibgpu_ctx *ctx, float *d_params, float *d_m, float *d_v
   if (rc) return rc;
   rc = launch_adam(V, d_params, d_grad, d_m, d_v, step, lr, true);
   if (rc) return rc;
-  return kernel_error_check(V.aux_err, V.stream);
+  return kernel_error_check(V);
 }
 
 int ibgpu_mlp_adam(ibgpu_ctx *ctx, float *d_params, const float *d_grad, float *d_m, float *d_v,
@@ -1524,7 +1520,7 @@ int ibgpu_tag_mesh(ibgpu_ctx *ctx, const ibgpu_tag_rule *rule, const float *d_pa
   uint8_t *rows = nullptr;
   if ((rc = tag_mesh_enqueue(ctx, rule, d_params, V.stream, &rows))) return rc;
   CKI(cudaMemcpyAsync(tags, rows, (size_t)V.ncells, cudaMemcpyDeviceToHost, V.stream));
-  if (d_params) return kernel_error_check(V.aux_err, V.stream);
+  if (d_params) return kernel_error_check(V);
   CKI(cudaStreamSynchronize(V.stream));
   return IBGPU_OK;
 }

@@ -195,8 +195,8 @@ def make_tag_rule(rule: dict) -> TagRule:
         if hasattr(ctype, "_length_"):
             arr = getattr(r, name)
             vals = np.asarray(v).ravel()
-            for k in range(min(len(vals), ctype._length_)):
-                arr[k] = vals[k].item()
+            n = min(len(vals), ctype._length_)
+            arr[:n] = vals[:n].tolist()
         else:
             setattr(r, name, v.item() if hasattr(v, "item") else v)
     return r
