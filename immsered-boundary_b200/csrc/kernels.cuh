@@ -45,6 +45,14 @@ __device__ __forceinline__ void step_reset(const StageArgs &a) {
 template <typename R>
 constexpr bool kPairFaces = sizeof(R) == 4;
 
+// How a stage CTA's warps share the halo.  FP64: half a record (two fields) per
+// lane, two warps per side, so that every warp waits for the same loads, and
+// dt through shared memory (20 steps at 2048^2 12.02 -> 11.78 ms, at 464^2
+// 0.655 -> 0.640).  FP32: a record per lane, one warp per side (7.99 ms
+// against 8.11 with half records: its stores are half as wide).
+template <typename R>
+constexpr bool kHalfHalo = sizeof(R) == 8;
+
 template <typename R>
 struct StageThreads {
   static constexpr int value = sizeof(R) == 8 ? 288 : kTileCells;
@@ -345,6 +353,10 @@ struct SRec<float> {
   static __device__ __forceinline__ void st(V *a, int i, int, float x, float y, float z, float w) {
     a[i] = make_float4(x, y, z, w);
   }
+  // half h of record i: components 2h, 2h + 1
+  static __device__ __forceinline__ void st_half(V *a, int i, int, int h, float x, float y) {
+    reinterpret_cast<float2 *>(a + i)[h] = make_float2(x, y);
+  }
 };
 
 template <>
@@ -359,6 +371,9 @@ struct SRec<double> {
                                             double w) {
     a[i] = make_double2(x, y);
     a[i + n] = make_double2(z, w);
+  }
+  static __device__ __forceinline__ void st_half(V *a, int i, int n, int h, double x, double y) {
+    a[i + h * n] = make_double2(x, y);
   }
 };
 
@@ -454,7 +469,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
                                            const CaseConst &cc, const LevelConst &L,
                                            const int tile, const int nb, const int phase,
                                            const int fold, typename SRec<R>::V *sq, uint8_t *sfl,
-                                           typename SRec<R>::V *fx, typename SRec<R>::V *fy) {
+                                           typename SRec<R>::V *fx, typename SRec<R>::V *fy,
+                                           double *sdt) {
   using S = SRec<R>;
   using V = typename S::V;
   constexpr int kFX = kTile + 1;  // faces of a row
@@ -466,12 +482,64 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
   // lane of the edge warp, negative on the others
   const int et = NT > kTileCells ? tid - kTileCells : (tid < 32 ? tid : -1);
 
-  // ---- the region: each thread its own cell, and four whole warps one side
-  //      of the two-cell halo each (south, north, west, east)
+  // ---- the region: each thread its own cell, and its lane's part of the
+  //      two-cell halo (kHalfHalo)
   const int rc = (ty + kHalo) * kReg + (tx + kHalo);
   Q4<R> c = {R(0), R(0), R(0), R(0)};
   uint8_t fown = 0;
-  {
+  if constexpr (kHalfHalo<R>) {
+    if (own) {
+      const int side = tid >> 6, half = (tid >> 4) & 1;
+      const int i = ((tid >> 1) & 16) + (tid & 15);  // this lane's cell of the side's 32
+      int x, y, hr;  // position in the neighbour tile, record in the region
+      if (side < 2) {
+        x = i & 15;
+        y = (side ? 0 : kTile - kHalo) + (i >> 4);
+        hr = ((i >> 4) + (side ? kTile + kHalo : 0)) * kReg + x + kHalo;
+      } else {
+        x = (side == 2 ? kTile - kHalo : 0) + (i & 1);
+        y = i >> 1;
+        hr = (y + kHalo) * kReg + (i & 1) + (side == 2 ? 0 : kTile + kHalo);
+      }
+      const int64_t hs = (int64_t)nb * kTileCells + y * kTile + x;
+      const int64_t os = (int64_t)tile * kTileCells + tid;
+      const TI *in0 = static_cast<const TI *>(v.sin[0]), *in1 = static_cast<const TI *>(v.sin[1]),
+               *in2 = static_cast<const TI *>(v.sin[2]), *in3 = static_cast<const TI *>(v.sin[3]);
+      const TI *ha = half ? in2 : in0, *hb = half ? in3 : in1;
+      R h0 = R(0), h1 = R(0);
+      if (UNI) {
+        // every load before the first store
+        c = Q4<R>{(R)in0[os], (R)in1[os], (R)in2[os], (R)in3[os]};
+        h0 = (R)ha[hs];
+        h1 = (R)hb[hs];
+      } else {
+        // presence flags first, then the state of the present cells: the
+        // stage input where the stages write it, else the step state
+        fown = a.flags[os];
+        const uint8_t fh = nb >= 0 ? a.flags[hs] : (uint8_t)0;
+        if (fown & CF_PRESENT) {
+          if (fown & (CF_PRIM | CF_RESET))
+            c = Q4<R>{(R)in0[os], (R)in1[os], (R)in2[os], (R)in3[os]};
+          else
+            c = Q4<R>{(R)a.s0[F_RHO][os], (R)a.s0[F_U][os], (R)a.s0[F_V][os], (R)a.s0[F_P][os]};
+        }
+        if (fh & CF_PRESENT) {
+          if (fh & (CF_PRIM | CF_RESET)) {
+            h0 = (R)ha[hs];
+            h1 = (R)hb[hs];
+          } else {
+            h0 = (R)a.s0[half ? F_V : F_RHO][hs];
+            h1 = (R)a.s0[half ? F_P : F_U][hs];
+          }
+        }
+        sfl[rc] = fown;
+        if (!half) sfl[hr] = fh;
+      }
+      S::st(sq, rc, NQ, c.x, c.y, c.z, c.w);
+      S::st_half(sq, hr, NQ, half, h0, h1);
+    }
+    if (tid == 0) *sdt = a.diag->dt;  // read by all after the faces
+  } else {
     const int side = (NT >> 5) - 1 - (tid >> 5), i = tid & 31;
     int64_t hs = -1;  // this lane's halo cell
     int hr = 0;
@@ -628,7 +696,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
         if (VISC && c > 0 && sizeof(R) == 8) res[c] += a.vsd[(int64_t)(c - 1) * a.nslots + slot];
       }
     }
-    const double dt = a.diag->dt;
+    const double dt = kHalfHalo<R> ? *sdt : a.diag->dt;
     const double scale = (v.tp * dt) * L.step_num * L.inv_vol;
     double nrho, nu, nv, np, ne, nT;
     bool wrote = false;
@@ -704,6 +772,7 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
   constexpr int NQ = kReg * kReg, NF = kTile * kFX;
   __shared__ V sq[S::kPlanes * NQ];
   __shared__ uint8_t sfl[NQ];
+  __shared__ double sdt;
   // face (i, j) between cells i-1 and i of row j at j*17 + i, between cells
   // j-1 and j of column i at j*16 + i: the lower cell's state, then the flux
   __shared__ V fx[S::kPlanes * NF];
@@ -717,10 +786,10 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
   // recover their primitives, so no presence flags or one-sided stencils
   const bool uni = a.tile_uniform != nullptr && a.tile_uniform[tile] != 0;
 
-  // this lane's side of the halo (south, north, west, east: four whole warps),
+  // this lane's side of the halo (south, north, west, east),
   // looked up beside the tile's level and uniform flag, so that the region's
   // loads wait for one round trip
-  const int side = (NT >> 5) - 1 - (tid >> 5);
+  const int side = kHalfHalo<R> ? tid >> 6 : (NT >> 5) - 1 - (tid >> 5);
   const int nb = side < 4 ? __ldg(a.tile_nb + (int64_t)tile * 9 +
                                   (side == 0 ? 1 : side == 1 ? 7 : side == 2 ? 3 : 5))
                           : -1;
@@ -745,8 +814,8 @@ __device__ __forceinline__ void stage_tile_fast(const StageArgs &a, const StageV
   }
 
   step_reset(a);
-  if (uni) stage_tile<R, LIM, VISC, FINAL, TI, NT, true>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
-  else stage_tile<R, LIM, VISC, FINAL, TI, NT, false>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy);
+  if (uni) stage_tile<R, LIM, VISC, FINAL, TI, NT, true>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy, &sdt);
+  else stage_tile<R, LIM, VISC, FINAL, TI, NT, false>(a, v, cc, L, tile, nb, phase, fold, sq, sfl, fx, fy, &sdt);
 }
 
 // TI: element type of the stage input (the FP64 step state for the first
