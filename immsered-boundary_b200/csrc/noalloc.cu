@@ -155,10 +155,13 @@ __global__ void __launch_bounds__(kTileCells)
 
 // tiled SoA -> caller rows
 __global__ void noalloc_rows_out_kernel(const double *s0, int nx, int ny, double *rows,
-                                        const DevDiag *diag, DevDiag *out) {
+                                        const DevDiag *diag, DevDiag *out, int *done) {
   dep_begin();
   dep_wait();
-  if (blockIdx.x == 0 && threadIdx.x == 0) *out = *diag;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *out = *diag;
+    *done = 0;  // also after calls that a caller let overlap
+  }
   const int64_t n = (int64_t)nx * ny;
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n;
        c += (int64_t)gridDim.x * blockDim.x) {
@@ -283,7 +286,7 @@ extern "C" int ibgpu_step_periodic_noalloc(const ibgpu_case *cs, int ts, int nx,
     else fast::launch_stage(sa, cc, ntiles, cs->limiter, false, fin, mixed, k, st, k > 0);
   }
   launch_dep(true, st, (nx * ny + 255) / 256, 256, noalloc_rows_out_kernel, d_s0, nx, ny,
-             d_rows_out, d_diag, m_page ? m_page : d_diag);
+             d_rows_out, d_diag, m_page ? m_page : d_diag, d_done);
   NA_CK(cudaGetLastError());
 
   DevDiag hd;
