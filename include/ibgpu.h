@@ -443,13 +443,13 @@ void ibgpu_destroy(ibgpu_ctx *ctx);
 /* ---------------------------------------------------------------------------
  * Batched independent cases (no counterpart in the reference, which runs one
  * case per process): several contexts, each with its own mesh, state and
- * case constants, advance together.  Every step runs each case's ghost
- * fills and viscous pass, one CFL launch over the cases whose pass is due,
- * then ONE persistent launch per stage covering the marching tiles of all
- * cases (a work list of (case, tile) pairs per subcycling phase, cases
- * interleaved).  The whole step is captured once per schedule phase in a
- * CUDA graph (the cases' ghost fills on parallel branches) and replayed;
- * the captures happen at the start of the first run.  On the first run an
+ * case constants, advance together.  Every step runs the ghost fills and the
+ * viscous pass, each launch over all cases it is due for, one CFL launch over
+ * the cases whose pass is due, then ONE launch per stage covering the
+ * marching tiles of all cases (a work list of (case, tile) pairs per
+ * subcycling phase, cases interleaved).  The whole step is captured once per
+ * schedule phase in a CUDA graph and replayed; the captures happen at the
+ * start of the first run.  On the first run an
  * autotuner times the candidate shapes of the merged stage launch (CTA
  * count: one CTA per work item or 1-4 / 1-6 persistent CTAs per SM; block:
  * 256 or 288 threads) and keeps the fastest.  The cases must agree on precision (IBGPU_FP64 or
