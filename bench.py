@@ -869,6 +869,8 @@ def config4_section(ib, wl, ind, stream, ncases: int, steps: int, warm: int = 4)
     indicator and by the plain criterion."""
     import numpy as np
     import torch
+    if not os.path.exists(os.path.join(ROOT, "oracle", "_ref", "ref_naca_minmod")):
+        return None  # the meshes come from the reference's own mesh generation
     envs = config4_cases()[:ncases]
     t0 = time.perf_counter()
     recs = config4_meshes(envs, host_workers(1.5e9))
