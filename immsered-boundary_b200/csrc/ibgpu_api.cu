@@ -729,7 +729,9 @@ int ibgpu_upload_topology(ibgpu_ctx *ctx, const ibgpu_cells *cells) {
     return rc;
   for (int f = 0; f < kStateFields; ++f)
     if ((rc = keep_alloc(ctx, &ctx->d_s0[f], (size_t)nslots))) return rc;
-  const size_t buf_elem = cs.precision == IBGPU_MIXED ? sizeof(float) : sizeof(double);
+  // (a one-stage scheme keeps its FP64 input there, see stage_args)
+  const size_t buf_elem =
+      cs.precision == IBGPU_MIXED && cs.nstages > 1 ? sizeof(float) : sizeof(double);
   for (int b = 0; b < 2; ++b)
     for (int f = 0; f < 4; ++f)
       if ((rc = keep_alloc(ctx, (unsigned char **)&ctx->d_buf[b][f], (size_t)nslots * buf_elem))) return rc;
@@ -1250,7 +1252,9 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
 }
 
 // Stage arguments of stage k (ping-pong stage buffers; the final stage
-// writes the step state).
+// writes the step state).  The only stage of a one-stage scheme reads a copy
+// of the state (stage_input_kernel) in the first buffer: neighbouring CTAs
+// read what it overwrites.
 void stage_args(const ibgpu_ctx *ctx, int k, StageArgs &sa) {
   const ibgpu_case &cs = ctx->cs;
   std::memset(&sa, 0, sizeof(sa));
@@ -1267,6 +1271,10 @@ void stage_args(const ibgpu_ctx *ctx, int k, StageArgs &sa) {
   for (int f = 0; f < 4; ++f) {
     sa.v.sin[f] = (k == 0) ? ctx->d_s0[map[f]] : ctx->d_buf[(k - 1) & 1][f];
     sa.v.sout[f] = fin ? nullptr : ctx->d_buf[k & 1][f];
+    if (cs.nstages == 1) {
+      sa.v.sin[f] = ctx->d_buf[0][f];
+      sa.v.sout[f] = ctx->d_buf[1][f];  // written by a batch's tuning runs only
+    }
   }
   sa.v.tp = cs.tp[k];
   // one wave of resident stage CTAs (4 per SM FP64, 5 mixed)
@@ -1356,6 +1364,11 @@ static int enqueue_stages(ibgpu_ctx *ctx, int ts, int step, bool fold_next, cuda
           sa.tile_begin = ctx->level_tile_begin[l0];
           const int nt = ctx->level_tile_begin[l1 - 1] + ctx->level_tile_count[l1 - 1] - sa.tile_begin;
           if (nt <= 0) return (int)IBGPU_OK;
+          if (cs.nstages == 1) {
+            if (exact) exact::launch_stage_input(sa, nt, st, dep);
+            else fast::launch_stage_input(sa, nt, st, dep);
+            dep = true;
+          }
           cudaEvent_t e = tm.mark(0);
           if (exact) exact::launch_stage(sa, ctx->cc, nt, cs.limiter, cs.viscous != 0, fin, false, k, st, dep);
           else fast::launch_stage(sa, ctx->cc, nt, cs.limiter, cs.viscous != 0, fin, mixed, k, st, dep);
@@ -1584,6 +1597,7 @@ int enqueue_batch_stages(ibgpu_batch *b, int r, int cfl, cudaStream_t st) {
     fast::launch_take_folded_batch(b->d_args, b->d_ccs, (int)b->cases.size(), b->nstages, st);
     CK(cudaGetLastError());
   }
+  if (b->nstages == 1) fast::launch_stage_input_batch(b->d_args, b->d_work[r], b->nwork[r], st);
   for (int k = 0; k < b->nstages; ++k) {
     fast::launch_stage_batch(b->d_args, b->d_ccs, b->d_work[r], b->nwork[r], k, b->nstages,
                              b->d_phase_base, b->limiter, b->visc, k == b->nstages - 1, b->mixed,
@@ -1593,10 +1607,6 @@ int enqueue_batch_stages(ibgpu_batch *b, int r, int cfl, cudaStream_t st) {
   return IBGPU_OK;
 }
 
-// Autotuner: time the first stage of the largest phase's work list at each
-// candidate CTA count (one CTA per item, or 1..6 resident CTAs per SM) and
-// keep the fastest.  Runs before the run's diag is initialised; it writes
-// only the first stage buffer, which stage 0 of every step rewrites.
 // Threads per CTA of the merged stage launch by default: 288 for FP64 (a
 // ninth warp owns the tile's edge faces), 256 for the mixed build.
 int default_threads(const ibgpu_batch *b) { return b->mixed ? kTileCells : kTileCells + 32; }
@@ -1604,7 +1614,9 @@ int default_threads(const ibgpu_batch *b) { return b->mixed ? kTileCells : kTile
 // The merged stage launch's shape from timed candidates on the busiest
 // phase's work list: the CTA count (one CTA per work item, or 1..4 (FP64) /
 // 1..6 (mixed) persistent CTAs per SM) and the block (256 or 288 threads),
-// each unless the caller fixed it.
+// each unless the caller fixed it.  Times the first stage, as a non-final one
+// also where it is the only one: it runs before the run's diag is initialised
+// and writes only a stage buffer, which every step rewrites.
 int autotune(ibgpu_batch *b) {
   int r = 0;
   for (int i = 1; i < b->period; ++i)
@@ -1639,13 +1651,15 @@ int autotune(ibgpu_batch *b) {
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
   int best_grid = grids[0], best_threads = blocks[0];
+  if (b->nstages == 1)
+    fast::launch_stage_input_batch(b->d_args, b->d_work[r], b->nwork[r], b->stream);
   for (int nt : blocks)
     for (int g : grids) {
       float tbest = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
         CK(cudaEventRecord(e0, b->stream));
         fast::launch_stage_batch(b->d_args, b->d_ccs, b->d_work[r], b->nwork[r], 0, b->nstages,
-                                 b->d_phase_base, b->limiter, b->visc, b->nstages == 1, b->mixed,
+                                 b->d_phase_base, b->limiter, b->visc, false, b->mixed,
                                  g, nt, b->table, b->stream);
         CK(cudaGetLastError());
         CK(cudaEventRecord(e1, b->stream));

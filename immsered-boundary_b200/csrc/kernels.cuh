@@ -884,6 +884,23 @@ __global__ void __launch_bounds__(NT, stage_min_blocks<R, NT>())
   }
 }
 
+// Input of a one-stage scheme's only stage.  That stage is first and final: it
+// writes rho, u, v, p of the step state, which its neighbours' CTAs read as
+// their halo, so it reads a copy of them made here (two passes over four
+// fields that schemes of several stages do not take).
+__device__ __forceinline__ void stage_input(const StageArgs &a, int tile) {
+  dep_begin();
+  dep_wait();
+  const int64_t s = (int64_t)tile * kTileCells + threadIdx.x;
+  constexpr int kMap[4] = {F_RHO, F_U, F_V, F_P};
+#pragma unroll
+  for (int f = 0; f < 4; ++f)
+    static_cast<double *>(const_cast<void *>(a.v.sin[f]))[s] = a.s0[kMap[f]][s];
+}
+__global__ void __launch_bounds__(kTileCells) stage_input_kernel(StageArgs a) {
+  stage_input(a, a.tile_begin + blockIdx.x);
+}
+
 // CFL time step over the normal cells of every level, NS_Solver::Comptdt
 // (NS_Solver.cpp:196-280): a per-cell bound, a warp-shuffle and block min and
 // one atomic per block (positive doubles order like their bit patterns).
@@ -1071,7 +1088,22 @@ void launch_stage(const StageArgs &a, const CaseConst &cc, int ntiles, int limit
   }
 }
 
+void launch_stage_input(const StageArgs &a, int ntiles, cudaStream_t st, bool dep) {
+  if (ntiles > 0) launch_dep(dep, st, ntiles, kTileCells, stage_input_kernel, a);
+}
+
 #ifdef IBGPU_FAST_BUILD
+// the same over a batch's work list (one-stage schemes: one StageArgs a case)
+__global__ void __launch_bounds__(kTileCells)
+    stage_input_batch(const StageArgs *__restrict__ args, const int2 *__restrict__ work) {
+  const int2 it = work[blockIdx.x];
+  stage_input(args[it.x], it.y);
+}
+void launch_stage_input_batch(const StageArgs *args, const int2 *work, int nwork,
+                              cudaStream_t st) {
+  if (nwork > 0) launch_dep(true, st, nwork, kTileCells, stage_input_batch, args, work);
+}
+
 template <typename R, int LIM, bool LOOP, bool TABLE, typename TI, int NT>
 static void launch_batch_n(const StageArgs *args, const CaseConst *ccs, const int2 *work, int nwork,
                            int stage, int nstages, const int *phase_base, bool visc,

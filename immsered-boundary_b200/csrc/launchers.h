@@ -18,6 +18,7 @@ namespace ibgpu {
   void launch_stage(const StageArgs &a, const CaseConst &cc, int ntiles, int limiter,         \
                     bool visc, bool final_stage, bool mixed, int stage, cudaStream_t st,      \
                     bool dep);                                                                \
+  void launch_stage_input(const StageArgs &a, int ntiles, cudaStream_t st, bool dep);         \
   void launch_cfl(const CflArgs &a, const CaseConst &cc, int nsm, cudaStream_t st, bool dep); \
   void launch_step_begin(DevDiag *d, cudaStream_t st, bool dep);                               \
   void launch_take_folded_cfl(DevDiag *d, const CaseConst &cc, cudaStream_t st, bool dep);    \
@@ -52,6 +53,7 @@ void launch_stage_batch(const StageArgs *args, const CaseConst *ccs, const int2 
                         int stage, int nstages, const int *phase_base, int limiter, bool visc,
                         bool final_stage, bool mixed, int grid, int threads, int table,
                         cudaStream_t st);
+void launch_stage_input_batch(const StageArgs *args, const int2 *work, int nwork, cudaStream_t st);
 // constant-memory table of batched stage arguments: reserve a byte range on
 // a device (16-byte aligned offset, -1 when it does not fit), release it,
 // write bytes at an offset (current device; blocking)

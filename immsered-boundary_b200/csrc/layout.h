@@ -80,7 +80,8 @@ struct DevDiag {
 constexpr int kHaloStage = 2;
 
 // Stage-dependent part of the stage arguments.  Stage input and output of
-// the varying cells (rho u v p): the first stage reads the FP64 step state;
+// the varying cells (rho u v p): the first stage reads the FP64 step state (the
+// only stage of a one-stage scheme a copy of it);
 // the stage buffers between stages hold FP64 values in the FP64 builds and
 // FP32 values in the mixed build, whose flux reads its inputs as FP32 (the
 // rounding happens at the store instead of the load: same values).

@@ -75,14 +75,16 @@ __device__ __forceinline__ int64_t tiled_slot(int ix, int iy, int ntx) {
 // tile grid, all-leaf flags, and its cells from the caller's rows (row-major
 // cells, FlowVariables layout) into the tiled SoA; with cfl also the tile's
 // CFL bound and first failing cell.  The last CTA to finish sets the step's
-// diagnostics and dt (NS_Solver::Comptdt) from the tiles'.  A small grid's
+// diagnostics and dt (NS_Solver::Comptdt) from the tiles'.  in1: null, or the
+// input of a one-stage scheme's stage (rho, u, v, p, which the stage cannot
+// read from the state it writes).  A small grid's
 // step is launches and little else: this one stands for four (set-up, rows,
 // CFL pass, dt): a step of 64 x 48 cells 74 -> 46 us, with the diagnostics
 // returned through a mapped page instead of a pageable copy.
 __global__ void __launch_bounds__(kTileCells)
     noalloc_load_kernel(const double *rows, int nx, int ntx, int nty, int32_t *nb, int32_t *lvl,
                         uint8_t *uniform, uint8_t *flags, double *s0, DevDiag *diag, int *done,
-                        unsigned long long *top, double dt, int cfl, CaseConst cc) {
+                        unsigned long long *top, double *in1, double dt, int cfl, CaseConst cc) {
   __shared__ unsigned long long sred[2 * (kTileCells / 32)];
   __shared__ int last;
   const int tile = blockIdx.x, tid = threadIdx.x;
@@ -106,6 +108,12 @@ __global__ void __launch_bounds__(kTileCells)
   s0[F_P * (int64_t)kMaxCells + s] = r[4];
   s0[F_E * (int64_t)kMaxCells + s] = r[6];
   s0[F_T * (int64_t)kMaxCells + s] = T;
+  if (in1) {
+    in1[s] = r[0];
+    in1[kMaxCells + s] = u;
+    in1[2 * kMaxCells + s] = v;
+    in1[3 * kMaxCells + s] = r[4];
+  }
   const unsigned long long none = (unsigned long long)__double_as_longlong(10000.0);
   unsigned long long best = none, bad = ~0ull;
   // block minima of both words, valid in thread 0
@@ -254,7 +262,8 @@ extern "C" int ibgpu_step_periodic_noalloc(const ibgpu_case *cs, int ts, int nx,
   int *d_done = (int *)(base + kOffDone);
   unsigned long long *d_top = (unsigned long long *)(base + kOffTop);
   launch_dep(false, st, ntiles, kTileCells, noalloc_load_kernel, d_rows_in, nx, ntx, nty, d_nb,
-             d_lvl, d_uniform, d_flags, d_s0, d_diag, d_done, d_top, *dt,
+             d_lvl, d_uniform, d_flags, d_s0, d_diag, d_done, d_top,
+             cs->nstages == 1 ? d_buf : (double *)nullptr, *dt,
              ts % cs->dt_var_step == 0 ? 1 : 0, cc);
   NA_CK(cudaGetLastError());
 
@@ -276,6 +285,7 @@ extern "C" int ibgpu_step_periodic_noalloc(const ibgpu_case *cs, int ts, int nx,
       // stage buffers (FP32 values in the mixed build, in the same regions)
       sa.v.sin[f] = (k == 0) ? (const void *)sa.s0[map[f]]
                              : (const void *)(d_buf + ((int64_t)(((k - 1) & 1) * 4 + f)) * kMaxCells);
+      if (cs->nstages == 1) sa.v.sin[f] = d_buf + (int64_t)f * kMaxCells;  // the load's in1
       sa.v.sout[f] = fin ? nullptr : (void *)(d_buf + ((int64_t)((k & 1) * 4 + f)) * kMaxCells);
     }
     sa.v.tp = cs->tp[k];
