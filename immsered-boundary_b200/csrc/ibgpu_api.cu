@@ -142,6 +142,8 @@ struct ibgpu_ctx {
     }
   };
   DevPairs res, pro;
+  // counts the uploads of lists (interfaces, boundaries, immersed cells)
+  uint64_t lists = 0;
 
   // domain ghosts: level-sorted, dependency waves [begin, end)
   int32_t *d_bc_ghost = nullptr, *d_bc_ref = nullptr, *d_bc_type = nullptr, *d_bc_face = nullptr;
@@ -1510,6 +1512,7 @@ struct ibgpu_batch {
     int n;
   };
   std::vector<std::vector<Fill>> fills;
+  std::vector<uint64_t> lists;     // the cases' ibgpu_ctx::lists they were built from
   int2 *d_fill_blocks = nullptr;  // every phase's (phases share equal lists)
   BatchPairs *d_pairs = nullptr;
   BatchBc *d_bcs = nullptr;
@@ -1546,17 +1549,22 @@ struct ibgpu_batch {
     graphs.clear();
     graphs_ready = false;
   }
-  void release() {
-    drop_graphs();
+  void drop_fills() {
     cudaFree(d_fill_blocks);
     d_fill_blocks = nullptr;
     fills.clear();
+    lists.clear();
     cudaFree(d_pairs);
     cudaFree(d_bcs);
     cudaFree(d_ibs);
     d_pairs = nullptr;
     d_bcs = nullptr;
     d_ibs = nullptr;
+    n_ibs = most_ib = 0;
+  }
+  void release() {
+    drop_graphs();
+    drop_fills();
     for (auto w : d_work) cudaFree(w);
     d_work.clear();
     cudaFree(d_cfl_work);
@@ -1774,8 +1782,10 @@ int build_fills(ibgpu_batch *b) {
   std::vector<int2> blocks;
   const int n = (int)b->cases.size();
   b->fills.assign(b->full_period, {});
+  b->lists.clear();
   for (int i = 0; i < n; ++i) {
     ibgpu_ctx *c = b->cases[i];
+    b->lists.push_back(c->lists);
     if (c->n_ib <= 0) continue;
     ibs.push_back(BatchIb{ib_args(c, 0, b->d_phase_base), i});
     b->most_ib = std::max(b->most_ib, c->n_ib);
@@ -1839,6 +1849,20 @@ int build_fills(ibgpu_batch *b) {
   CK(cudaMemcpy(b->d_bcs, bcs.data(), bcs.size() * sizeof(BatchBc), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(b->d_ibs, ibs.data(), ibs.size() * sizeof(BatchIb), cudaMemcpyHostToDevice));
   return IBGPU_OK;
+}
+
+// The lists follow the cases' own: new ones since they were built (which left
+// the old arrays freed) are taken up, and the captured steps made anew.
+int update_fills(ibgpu_batch *b) {
+  bool same = b->lists.size() == b->cases.size();
+  for (size_t i = 0; same && i < b->cases.size(); ++i) same = b->lists[i] == b->cases[i]->lists;
+  if (same) return IBGPU_OK;
+  if (b->stream) CK(cudaStreamSynchronize(b->stream));
+  b->drop_graphs();
+  b->drop_fills();
+  const int rc = build_fills(b);
+  if (rc) b->drop_fills();
+  return rc;
 }
 
 // The graph of one whole batch step, captured on first use: nothing in it
@@ -2069,6 +2093,7 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
   // rarely, take each case's own launches
   bool merged = b->full_period <= kMaxBatchPeriod;
   for (int i = 0; i < n; ++i) merged = merged && !b->cases[i]->timing;
+  if (merged && (rc = update_fills(b))) return rc;
   const bool use_graphs = merged && b->stream != nullptr && !b->timing;
   if (use_graphs && (rc = batch_prepare_graphs(b))) return rc;
   for (int i = 0; i < n; ++i) {
@@ -2263,6 +2288,7 @@ int ibgpu_upload_interfaces(ibgpu_ctx *ctx, const ibgpu_cf_pairs *pp) {
   const int nlev = ctx->cs.nlevels;
   cudaStream_t st = ctx->stream;
   CK(cudaStreamSynchronize(st));
+  ++ctx->lists;
   ctx->res.free();
   ctx->pro.free();
   // restriction: per coarse level, in list order
@@ -2357,6 +2383,7 @@ int ibgpu_upload_boundaries(ibgpu_ctx *ctx, const ibgpu_bc *bc) {
   const int nlev = ctx->cs.nlevels;
   cudaStream_t st = ctx->stream;
   CK(cudaStreamSynchronize(st));
+  ++ctx->lists;
   for (int32_t **p : {&ctx->d_bc_ghost, &ctx->d_bc_ref, &ctx->d_bc_type, &ctx->d_bc_face}) {
     cudaFree(*p);
     *p = nullptr;
@@ -2495,6 +2522,7 @@ int ibgpu_upload_ib(ibgpu_ctx *ctx, const ibgpu_ib *ib) {
   bool grows = false;
   for (const auto &q : need) grows = grows || q.second > ctx->cap[q.first];
   if (grows) CK(cudaStreamSynchronize(st));
+  ++ctx->lists;
   int e;
   if ((e = keep_upload(ctx, &ctx->d_ib_cell, cell, st)) || (e = keep_upload(ctx, &ctx->d_ib_intp, intp, st)) ||
       (e = keep_upload(ctx, &ctx->d_ib_f, cf, st)) || (e = keep_alloc(ctx, &ctx->d_ib_out, 6 * cell.size())) ||

@@ -457,9 +457,10 @@ void ibgpu_destroy(ibgpu_ctx *ctx);
  * intervals (dt_var_step) may differ when each divides the longest marching
  * step of the batch (each case then takes its CFL pass on its own steps, as
  * meshes of different depths do); the batch runs on the first context's
- * stream.  Uploads to a context (topology,
- * lists) invalidate a batch that holds it: destroy and recreate it.  A batch
- * is destroyed before any context it holds.
+ * stream.  A topology upload to a context invalidates a batch that holds it:
+ * destroy and recreate it.  Its lists (interfaces, boundaries, immersed
+ * cells) may be uploaded again between runs; the next run takes them up.  A
+ * batch is destroyed before any context it holds.
  * ------------------------------------------------------------------------- */
 typedef struct ibgpu_batch ibgpu_batch;
 int ibgpu_batch_create(ibgpu_ctx *const *cases, int ncases, ibgpu_batch **out);

@@ -1,0 +1,92 @@
+"""The lists of a context (coarse/fine pairs, domain ghosts, immersed cells)
+on their way into the fills' launches: what a step launches is what was
+uploaded last, and arrays that were freed are never passed on."""
+import os
+import struct
+import sys
+
+import pytest
+
+from conftest import GOLDEN_DIR, load_pkg
+from host_api import HostApi, words
+
+sys.path.insert(0, GOLDEN_DIR)
+import make_golden  # noqa: E402
+
+wl = load_pkg().workloads
+
+
+@pytest.fixture(scope="module")
+def api(tmp_path_factory):
+    return HostApi(str(tmp_path_factory.mktemp("host")))
+
+
+@pytest.fixture(scope="module")
+def record():
+    return make_golden.load("naca_minmod_s4_n64_l3")
+
+
+def upload(s, L, which=("cf", "bc", "ib"), backpressure=None, bc=None, ib=None):
+    if "cf" in which:
+        s.upload_interfaces(L["res"], L["pro"])
+    if "bc" in which:
+        n = len(L["bc"]) if bc is None else bc
+        s.upload_boundaries(L["bc"][:n], L["bc_nmv"][:n], L["facevar"],
+                            L["bc_scalars"][0] if backpressure is None else backpressure,
+                            L["bc_scalars"][1])
+    if "ib" in which:
+        n = len(L["ib"]) if ib is None else ib
+        s.upload_ib(L["ib"][:n], L["ib_f"][:n], L["patch"], L["patch_f"], L["body_center"])
+
+
+def solver(api, record, precision="FP64"):
+    L = wl.naca_lists(record, 0)
+    s = api.ib.FlowSolver(wl.naca_params(record, 0, getattr(api.ib, precision)))
+    s.upload_topology(L["level"], L["ix"], L["iy"], L["flags"])
+    upload(s, L)
+    s.init_flow(L["prim"])
+    return s, L
+
+
+def low32(word):
+    return struct.unpack("<i", struct.pack("<q", word)[:4])[0]
+
+
+def as_double(word):
+    return struct.unpack("<d", struct.pack("<q", word))[0]
+
+
+# the first segment of a batched launch is the first case's
+def first_bc(api):
+    """(ghost pointer, backpressure) of BatchBc[0]"""
+    w = words(api.launches("bc_kernel_batch")[-1][2][0], 8)
+    return w[0], as_double(w[7])
+
+
+def first_ib(api):
+    """(cell pointer, cells) of BatchIb[0]"""
+    w = words(api.launches("ib_kernel_batch")[-1][2][0], 5)
+    return w[0], low32(w[4])
+
+
+def test_batch_takes_up_lists_uploaded_after_its_creation(api, record):
+    (a, L), (b, _) = solver(api, record), solver(api, record)
+    batch = api.ib.Batch([a, b])
+    for k, (pressure, nbc, nib) in enumerate([(0.25, 40, 30), (0.5, len(L["bc"]), len(L["ib"]))]):
+        upload(a, L, backpressure=pressure, bc=nbc, ib=nib)  # before the first run, and after it
+        api.clear()
+        batch.run(0, 4)
+        ghost, got = first_bc(api)
+        assert got == pressure and api.live(ghost)
+        cell, n = first_ib(api)
+        assert n == nib and api.live(cell)
+        for part in ("restrict_kernel_batch", "prolong_kernel_batch"):
+            seg = words(api.launches(part)[-1][2][0], 2)
+            assert api.live(seg[0]) and api.live(seg[1])
+        # unchanged lists: the captured steps serve
+        api.clear()
+        batch.run(4, 4)
+        assert not api.launches("bc_kernel_batch")
+    batch.close()
+    a.close()
+    b.close()
