@@ -135,7 +135,10 @@ __global__ void __launch_bounds__(kTileCells)
   if (cfl) {
     const double d0 = cfl_cell_bound(T, u, v, cc.lev[0], cc);
     if (d0 < 0.0) bad = error_key(1, ERR_CFL_NEG_DT, (int)s);
-    if (d0 < 10000.0) best = (unsigned long long)__double_as_longlong(d0);  // ignores NaN
+    // as the CFL pass's atomic minimum of bit patterns: a negative bound (its
+    // sign bit makes it large) or NaN leaves 10000
+    const unsigned long long b0 = (unsigned long long)__double_as_longlong(d0);
+    if (b0 < none) best = b0;
   }
   block_min();
   if (tid == 0) {
