@@ -2370,9 +2370,16 @@ int ibgpu_upload_interfaces(ibgpu_ctx *ctx, const ibgpu_cf_pairs *pp) {
     CK(cudaStreamSynchronize(st));  // the copies read the vectors above
     return IBGPU_OK;
   };
+  // both lists, or (when an allocation or a copy fails) none
+  ibgpu_ctx::DevPairs res, pro;
   int e;
-  if ((e = pack(ctx->res, rc_, rf, nullptr)) || (e = pack(ctx->pro, pc, pf, &pn))) return e;
-  CK(cudaStreamSynchronize(st));
+  if ((e = pack(res, rc_, rf, nullptr)) || (e = pack(pro, pc, pf, &pn))) {
+    res.free();
+    pro.free();
+    return e;
+  }
+  ctx->res = std::move(res);
+  ctx->pro = std::move(pro);
   return IBGPU_OK;
 }
 

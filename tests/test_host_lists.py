@@ -90,3 +90,33 @@ def test_batch_takes_up_lists_uploaded_after_its_creation(api, record):
     batch.close()
     a.close()
     b.close()
+
+
+def run_and_check_pointers(api, s, part, n):
+    """Four steps; every launch whose kernel's name contains `part` gets live
+    arrays in its first n arguments.  Returns the number of these launches."""
+    api.clear()
+    s.run(0, 4)
+    launches = api.launches(part)
+    assert api.launches("stage_kernel")
+    for name, _, w in launches:
+        assert all(api.live(p) for p in w[:n]), name
+    return len(launches)
+
+
+# five arrays: coarse, sons (and neighbours) of both lists
+@pytest.mark.parametrize("nth", range(1, 6))
+def test_failed_interface_upload_leaves_no_pairs(api, record, nth):
+    s, L = solver(api, record)
+    assert run_and_check_pointers(api, s, "restrict_kernel", 2)
+    assert run_and_check_pointers(api, s, "prolong_kernel", 3)
+    api.fail_malloc(nth)
+    with pytest.raises(api.ib.IbgpuError) as e:
+        upload(s, L, ("cf",))
+    api.fail_malloc(0)
+    assert e.value.code == api.ib.E_NOMEM
+    assert run_and_check_pointers(api, s, "restrict_kernel", 2) == 0
+    assert run_and_check_pointers(api, s, "prolong_kernel", 3) == 0
+    upload(s, L, ("cf",))
+    assert run_and_check_pointers(api, s, "restrict_kernel", 2)
+    s.close()
