@@ -2391,6 +2391,7 @@ int ibgpu_upload_boundaries(ibgpu_ctx *ctx, const ibgpu_bc *bc) {
   cudaStream_t st = ctx->stream;
   CK(cudaStreamSynchronize(st));
   ++ctx->lists;
+  ctx->bc_waves.clear();  // none until the new arrays are in place
   for (int32_t **p : {&ctx->d_bc_ghost, &ctx->d_bc_ref, &ctx->d_bc_type, &ctx->d_bc_face}) {
     cudaFree(*p);
     *p = nullptr;
@@ -2426,7 +2427,7 @@ int ibgpu_upload_boundaries(ibgpu_ctx *ctx, const ibgpu_bc *bc) {
   // dependency waves: a ghost whose reference is written earlier in the list
   // runs after that write; one written later must read it before the write;
   // a cell written twice keeps the later value (BCBoxTreat is sequential)
-  ctx->bc_waves.assign(nlev, {});
+  std::vector<std::vector<std::pair<int, int>>> waves(nlev);
   std::vector<int32_t> hg, hr, ht, hf;
   std::vector<double> hn;
   for (int l = 0; l < nlev; ++l) {
@@ -2450,7 +2451,7 @@ int ibgpu_upload_boundaries(ibgpu_ctx *ctx, const ibgpu_bc *bc) {
     while (i < E.size()) {
       size_t j = i;
       while (j < E.size() && E[j].wave == E[i].wave) ++j;
-      ctx->bc_waves[l].push_back({(int)(hg.size() + i), (int)(hg.size() + j)});
+      waves[l].push_back({(int)(hg.size() + i), (int)(hg.size() + j)});
       i = j;
     }
     for (auto &en : E) {
@@ -2471,6 +2472,7 @@ int ibgpu_upload_boundaries(ibgpu_ctx *ctx, const ibgpu_bc *bc) {
   ctx->cos_in = std::cos(bc->inlet_flow_angle);
   ctx->sin_in = std::sin(bc->inlet_flow_angle);
   CK(cudaStreamSynchronize(st));
+  ctx->bc_waves = std::move(waves);
   return IBGPU_OK;
 }
 

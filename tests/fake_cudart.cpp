@@ -12,7 +12,7 @@
 namespace {
 // bytes kept of a launch's first argument: what every one has on the caller's
 // stack, more of the stages' argument block
-constexpr size_t kArgBytes = 24, kStageBytes = 160;
+constexpr size_t kArgBytes = 48, kStageBytes = 160;
 struct Launch {
   std::string name;
   unsigned grid;

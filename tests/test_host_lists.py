@@ -120,3 +120,24 @@ def test_failed_interface_upload_leaves_no_pairs(api, record, nth):
     upload(s, L, ("cf",))
     assert run_and_check_pointers(api, s, "restrict_kernel", 2)
     s.close()
+
+
+# refused (an unknown type), or one of its six allocations fails
+@pytest.mark.parametrize("nth", range(7))
+def test_failed_boundary_upload_leaves_no_ghosts(api, record, nth):
+    s, L = solver(api, record)
+    assert run_and_check_pointers(api, s, "bc_kernel", 6)
+    if nth == 0:
+        bad = dict(L, bc=L["bc"].copy())
+        bad["bc"][-1, 6] = -3
+    else:
+        bad = L
+        api.fail_malloc(nth)
+    with pytest.raises(api.ib.IbgpuError) as e:
+        upload(s, bad, ("bc",))
+    api.fail_malloc(0)
+    assert e.value.code == (api.ib.E_NOMEM if nth else api.ib.E_ARG)
+    assert run_and_check_pointers(api, s, "bc_kernel", 6) == 0
+    upload(s, L, ("bc",))
+    assert run_and_check_pointers(api, s, "bc_kernel", 6)
+    s.close()
