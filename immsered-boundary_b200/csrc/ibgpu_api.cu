@@ -2532,6 +2532,7 @@ int ibgpu_upload_ib(ibgpu_ctx *ctx, const ibgpu_ib *ib) {
   for (const auto &q : need) grows = grows || q.second > ctx->cap[q.first];
   if (grows) CK(cudaStreamSynchronize(st));
   ++ctx->lists;
+  ctx->n_ib = ctx->n_pat = ctx->nbodies = 0;  // none until every buffer is in place
   int e;
   if ((e = keep_upload(ctx, &ctx->d_ib_cell, cell, st)) || (e = keep_upload(ctx, &ctx->d_ib_intp, intp, st)) ||
       (e = keep_upload(ctx, &ctx->d_ib_f, cf, st)) || (e = keep_alloc(ctx, &ctx->d_ib_out, 6 * cell.size())) ||

@@ -5,6 +5,7 @@ import os
 import struct
 import sys
 
+import numpy as np
 import pytest
 
 from conftest import GOLDEN_DIR, load_pkg
@@ -140,4 +141,24 @@ def test_failed_boundary_upload_leaves_no_ghosts(api, record, nth):
     assert run_and_check_pointers(api, s, "bc_kernel", 6) == 0
     upload(s, L, ("bc",))
     assert run_and_check_pointers(api, s, "bc_kernel", 6)
+    s.close()
+
+
+# eleven buffers, which longer lists make grow (all but the body's own three)
+@pytest.mark.parametrize("nth", range(1, 9))
+def test_failed_body_upload_leaves_no_cells(api, record, nth):
+    s, L = solver(api, record)
+    assert run_and_check_pointers(api, s, "ib_kernel", 4)
+    longer = dict(L, **{k: np.repeat(L[k], 2, 0) for k in ("ib", "ib_f", "patch", "patch_f")})
+    api.fail_malloc(nth)
+    with pytest.raises(api.ib.IbgpuError) as e:
+        upload(s, longer, ("ib",))
+    api.fail_malloc(0)
+    assert e.value.code == api.ib.E_NOMEM
+    assert run_and_check_pointers(api, s, "ib_", 4) == 0
+    api.clear()
+    s.wall_forces()
+    assert not api.launches("force")
+    upload(s, longer, ("ib",))
+    assert run_and_check_pointers(api, s, "ib_kernel", 4)
     s.close()
