@@ -16,6 +16,7 @@
 #include "cfl.cuh"
 #include "dependent.cuh"
 #include "flux.cuh"
+#include "cell_states.cuh"
 #include "layout.h"
 
 namespace ibgpu {
@@ -328,20 +329,6 @@ __global__ void __launch_bounds__(kTileCells) stage_kernel(StageArgs a, CaseCons
   }
 }
 
-// Four values of one cell (rho, u, v, p), one limited slope set, or one
-// face flux (mass, x-momentum, y-momentum, energy).  In shared memory an FP32
-// record is one float4; an FP64 record is split over two double2 planes
-// (components 0-1 at [i], 2-3 at [i + n] for an array of n records), so a
-// warp reading consecutive records moves 16-byte words at a 16-byte stride
-// and every 128-bit access is conflict-free.
-template <typename R>
-struct Q4 {
-  R x, y, z, w;
-};
-
-template <typename R>
-struct SRec;
-
 template <>
 struct SRec<float> {
   using V = float4;
@@ -376,48 +363,6 @@ struct SRec<double> {
     a[i + h * n] = make_double2(x, y);
   }
 };
-
-template <typename R>
-__device__ __forceinline__ Q4<R> add4(const Q4<R> &a, const Q4<R> &b) {
-  return Q4<R>{a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w};
-}
-template <typename R>
-__device__ __forceinline__ Q4<R> sub4(const Q4<R> &a, const Q4<R> &b) {
-  return Q4<R>{a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w};
-}
-
-// The states region cell rc (value c) gives to its two faces along `step`:
-// lo to the face towards rc - step, hi to the one towards rc + step.  A cell
-// whose neighbour on one side is missing has a flux only on the other, with
-// the reference's one-sided reconstruction (its stencil then takes the cell
-// two steps away on that side, NS_Solver.H:743-750); states of faces that
-// carry no flux are left unset (c).
-template <typename R, int LIM, int NQ>
-__device__ __forceinline__ void cell_states(const typename SRec<R>::V *sq, const uint8_t *sfl,
-                                            const Q4<R> &c, int rc, int step, bool uni, Q4<R> &lo,
-                                            Q4<R> &hi) {
-  using S = SRec<R>;
-  if (uni || ((sfl[rc - step] & CF_PRESENT) && (sfl[rc + step] & CF_PRESENT))) {
-    const Q4<R> m = S::ld(sq, rc - step, NQ), p = S::ld(sq, rc + step, NQ);
-    const Q4<R> s = {limited_slope<LIM>(c.x - m.x, p.x - c.x),
-                     limited_slope<LIM>(c.y - m.y, p.y - c.y),
-                     limited_slope<LIM>(c.z - m.z, p.z - c.z),
-                     limited_slope<LIM>(c.w - m.w, p.w - c.w)};
-    lo = sub4(c, s);
-    hi = add4(c, s);
-    return;
-  }
-  lo = hi = c;
-  if (sfl[rc - step] & CF_PRESENT) {
-    const Q4<R> m = S::ld(sq, rc - step, NQ), o = S::ld(sq, rc - 2 * step, NQ);
-    lo = Q4<R>{muscl_right_fast<LIM>(m.x, c.x, o.x), muscl_right_fast<LIM>(m.y, c.y, o.y),
-               muscl_right_fast<LIM>(m.z, c.z, o.z), muscl_right_fast<LIM>(m.w, c.w, o.w)};
-  } else if (sfl[rc + step] & CF_PRESENT) {
-    const Q4<R> p = S::ld(sq, rc + step, NQ), o = S::ld(sq, rc + 2 * step, NQ);
-    hi = Q4<R>{muscl_left_fast<LIM>(o.x, c.x, p.x), muscl_left_fast<LIM>(o.y, c.y, p.y),
-               muscl_left_fast<LIM>(o.z, c.z, p.z), muscl_left_fast<LIM>(o.w, c.w, p.w)};
-  }
-}
 
 // Whether the face between cells with flags fL | fR carries a flux.
 __device__ __forceinline__ bool face_active(uint8_t fL, uint8_t fR) {
@@ -594,9 +539,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
   Q4<R> wx = {}, wy = {}, we = {};  // own cell's state at its west / south face, edge cell's
   if (own) {
     Q4<R> hi;
-    cell_states<R, LIM, NQ>(sq, sfl, c, rc, 1, UNI, wx, hi);
+    cell_states<R, LIM, NQ, kLow | kHigh>(sq, sfl, c, rc, 1, UNI, wx, hi);
     S::st(fx, ty * kFX + tx + 1, NF, hi.x, hi.y, hi.z, hi.w);
-    cell_states<R, LIM, NQ>(sq, sfl, c, rc, kReg, UNI, wy, hi);
+    cell_states<R, LIM, NQ, kLow | kHigh>(sq, sfl, c, rc, kReg, UNI, wy, hi);
     S::st(fy, (ty + 1) * kTile + tx, NF, hi.x, hi.y, hi.z, hi.w);
   }
   const bool xd = et < 16;  // edge lanes: east column, then north row
@@ -607,9 +552,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const StageVar &v
     // its last face
     const int r0 = er - (kTile + 1) * estep;
     Q4<R> lo, hi;
-    cell_states<R, LIM, NQ>(sq, sfl, S::ld(sq, r0, NQ), r0, estep, UNI, lo, hi);
+    cell_states<R, LIM, NQ, kHigh>(sq, sfl, S::ld(sq, r0, NQ), r0, estep, UNI, lo, hi);
     S::st(xd ? fx : fy, xd ? ee * kFX : ee, NF, hi.x, hi.y, hi.z, hi.w);
-    cell_states<R, LIM, NQ>(sq, sfl, S::ld(sq, er, NQ), er, estep, UNI, we, hi);
+    cell_states<R, LIM, NQ, kLow>(sq, sfl, S::ld(sq, er, NQ), er, estep, UNI, we, hi);
   }
   __syncthreads();
 
