@@ -11,7 +11,6 @@
 #include <new>
 #include <string>
 #include <unordered_map>
-#include <unordered_set>
 #include <map>
 #include <numeric>
 #include <vector>
@@ -2350,13 +2349,16 @@ int ibgpu_upload_interfaces(ibgpu_ctx *ctx, const ibgpu_cf_pairs *pp) {
     for (int l = 0; l < nlev; ++l) {
       P.begin[l] = (int)ac.size();
       if (l > 0) {
-        const std::vector<int32_t> &wrote = nb ? f[l - 1] : c[l], &a1 = nb ? c[l] : f[l - 1];
-        std::unordered_set<int32_t> w(wrote.begin(), wrote.end());
-        bool free = true;
-        for (int32_t x : a1) free = free && !w.count(x);
-        if (nb)
-          for (int32_t x : (*nb)[l]) free = free && !w.count(x);
-        P.joins[l] = free;
+        // (all of them slots of level l: a bit each; a hash set of the written
+        // ones took a third of the call)
+        const std::vector<int32_t> &wrote = nb ? f[l - 1] : c[l], &read = nb ? c[l] : f[l - 1];
+        const int32_t s0 = ctx->level_tile_begin[l] * kTileCells;
+        std::vector<bool> w((size_t)ctx->level_tile_count[l] * kTileCells, false);
+        for (int32_t x : wrote) w[x - s0] = true;
+        auto clear_of = [&](const std::vector<int32_t> &v) {
+          return std::none_of(v.begin(), v.end(), [&](int32_t x) { return w[x - s0]; });
+        };
+        P.joins[l] = clear_of(read) && (!nb || clear_of((*nb)[l]));
       }
       ac.insert(ac.end(), c[l].begin(), c[l].end());
       af.insert(af.end(), f[l].begin(), f[l].end());
