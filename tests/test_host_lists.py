@@ -162,3 +162,68 @@ def test_failed_body_upload_leaves_no_cells(api, record, nth):
     upload(s, longer, ("ib",))
     assert run_and_check_pointers(api, s, "ib_kernel", 4)
     s.close()
+
+
+def chained_mesh(chained):
+    """Three levels of 40 x 40 cells whose level-1 pairs touch the cells that
+    the level-0 pairs read (restriction) and write (prolongation), or not."""
+    from test_gpu_interface_order import pair
+    cx = 6 if chained else 30
+    keys = np.array([(l, x, y) for l in range(3) for y in range(40) for x in range(40)], np.int32)
+    g = wl.gas_constants(0.5, 0.0)
+    P = dict(g, cfl=0.5, dt_ratio=1.0, dt_var_step=4, nstages=3, tp=wl.TP[3],
+             initvar=wl.freestream(g, 0.2), nlevels=3,
+             dh=[(0.4 / 2 ** l, 0.4 / 2 ** l, 0.1) for l in range(3)], march_step=[4, 2, 1],
+             march_left=[0, 0, 0], step_num=[4.0, 2.0, 1.0], average_step=[1, 1, 1],
+             average_left=[0, 0, 0], prolong_step=[1, 1, 1], prolong_left=[0, 0, 0],
+             domain_nx=64, domain_ny=64, dt0=1.0)
+    res = [pair(1, cx, 6, 20, 20), pair(0, 9, 9, 6, 6)]
+    pro = [pair(1, cx + 1, 11, 2, 2), pair(0, 17, 3, 6, 10)]
+    return P, keys.T, res, pro
+
+
+@pytest.mark.parametrize("chained", [True, False])
+def test_levels_share_a_fill_launch_only_when_independent(api, chained):
+    P, (lv, x, y), res, pro = chained_mesh(chained)
+    sols = []
+    for _ in range(2):
+        s = api.ib.FlowSolver(P)
+        s.upload_topology(lv, x, y, np.full(len(lv), api.ib.CELL_PRESENT, np.uint8))
+        s.upload_interfaces(np.array(res), np.array(pro))
+        s.init_flow(np.ones((len(lv), 7)))
+        sols.append(s)
+    pairs = [1, 1] if chained else [2]
+    api.clear()
+    sols[0].run(0, 1)
+    for part in ("restrict_kernel", "prolong_kernel"):
+        assert [low32(w[3]) for _, _, w in api.launches(part)] == pairs
+    # the k-th launch of every case in one: a block each
+    b = api.ib.Batch(sols)
+    api.clear()
+    b.run(0, 1)
+    for part in ("restrict_kernel_batch", "prolong_kernel_batch"):
+        grids = [g for _, g, _ in api.launches(part)]
+        assert grids[:len(pairs)] == [2] * len(pairs)
+    b.close()
+    for s in sols:
+        s.close()
+
+
+# one CTA takes 1024 immersed cells; more, two launches with the states between
+@pytest.mark.parametrize("n,kernels", [(1024, ["ib_kernel"]), (1025, ["ib_compute", "ib_store"])])
+def test_immersed_cells_choose_their_launches(api, record, n, kernels):
+    (a, L), (b, _) = solver(api, record), solver(api, record)
+    many = dict(L, ib=np.resize(L["ib"], (n, 18)), ib_f=np.resize(L["ib_f"], (n, 16)))
+    upload(a, many, ("ib",))
+    api.clear()
+    a.run(0, 1)
+    names = [name for name, _, _ in api.launches("ib_")]
+    assert len(names) == len(kernels) and all(k in m for k, m in zip(kernels, names))
+    batch = api.ib.Batch([a, b])
+    api.clear()
+    batch.run(0, 1)
+    assert bool(api.launches("ib_kernel_batch")) == (n <= 1024)
+    assert bool(api.launches("ib_compute")) == (n > 1024)
+    batch.close()
+    a.close()
+    b.close()
