@@ -1252,6 +1252,10 @@ int enqueue_prestage(ibgpu_ctx *ctx, int ts, int step, cudaStream_t st, RunTimer
   return IBGPU_OK;
 }
 
+// Threads per CTA of the stage launches by default: 288 for FP64 (a ninth
+// warp owns the tile's edge faces), 256 for the mixed build.
+int default_threads(bool mixed) { return mixed ? kTileCells : kTileCells + 32; }
+
 // Stage arguments of stage k (ping-pong stage buffers; the final stage
 // writes the step state).  The only stage of a one-stage scheme reads a copy
 // of the state (stage_input_kernel) in the first buffer: neighbouring CTAs
@@ -1278,8 +1282,9 @@ void stage_args(const ibgpu_ctx *ctx, int k, StageArgs &sa) {
     }
   }
   sa.v.tp = cs.tp[k];
-  // one wave of resident stage CTAs (4 per SM FP64, 5 mixed)
-  sa.prefetch = ctx->nsm * (cs.precision == IBGPU_MIXED ? 5 : 4);
+  // one wave of resident stage CTAs
+  const bool mixed = cs.precision == IBGPU_MIXED;
+  sa.prefetch = ctx->nsm * fast::stage_resident_ctas(mixed, default_threads(mixed));
 }
 
 int64_t marched_cells(const ibgpu_ctx *ctx, int ts) {
@@ -1614,13 +1619,9 @@ int enqueue_batch_stages(ibgpu_batch *b, int r, int cfl, cudaStream_t st) {
   return IBGPU_OK;
 }
 
-// Threads per CTA of the merged stage launch by default: 288 for FP64 (a
-// ninth warp owns the tile's edge faces), 256 for the mixed build.
-int default_threads(const ibgpu_batch *b) { return b->mixed ? kTileCells : kTileCells + 32; }
-
 // The merged stage launch's shape from timed candidates on the busiest
-// phase's work list: the CTA count (one CTA per work item, or 1..4 (FP64) /
-// 1..6 (mixed) persistent CTAs per SM) and the block (256 or 288 threads),
+// phase's work list: the CTA count (one CTA per work item, or one persistent
+// CTA per SM up to as many as are resident) and the block (256 or 288 threads),
 // each unless the caller fixed it.  Times the first stage, as a non-final one
 // also where it is the only one: it runs before the run's diag is initialised
 // and writes only a stage buffer, which every step rewrites.
@@ -1633,23 +1634,29 @@ int autotune(ibgpu_batch *b) {
   b->tune_ms.clear();
   if (b->nwork[r] == 0) {
     b->grid = std::max(b->fixed_grid, 0);
-    b->threads = b->fixed_threads ? b->fixed_threads : default_threads(b);
+    b->threads = b->fixed_threads ? b->fixed_threads : default_threads(b->mixed);
     b->tuned = true;
     return IBGPU_OK;
   }
-  std::vector<int> grids, blocks;
-  if (b->fixed_grid >= 0) {
-    grids.push_back(b->fixed_grid);
-  } else {
+  std::vector<int> blocks;
+  // (more persistent CTAs than are resident run as a partial second wave)
+  auto grids_of = [&](int threads) {
+    std::vector<int> grids;
+    if (b->fixed_grid >= 0) {
+      grids.push_back(b->fixed_grid);
+      return grids;
+    }
     grids.push_back(0);
-    for (int m = 1; m <= (b->mixed ? 6 : 4); ++m)
+    for (int m = 1; m <= fast::stage_resident_ctas(b->mixed, threads); ++m)
       if (m * b->nsm < b->nwork[r]) grids.push_back(m * b->nsm);
-  }
+    return grids;
+  };
   if (b->fixed_threads) blocks.push_back(b->fixed_threads);
-  else blocks = {default_threads(b), b->mixed ? kTileCells + 32 : kTileCells};
-  if (grids.size() * blocks.size() == 1) {
-    b->grid = grids[0];
-    b->threads = blocks[0];
+  else blocks = {default_threads(b->mixed), b->mixed ? kTileCells + 32 : kTileCells};
+  int best_grid = grids_of(blocks[0])[0], best_threads = blocks[0];
+  if (blocks.size() == 1 && grids_of(blocks[0]).size() == 1) {
+    b->grid = best_grid;
+    b->threads = best_threads;
     b->tuned = true;
     return IBGPU_OK;
   }
@@ -1657,11 +1664,10 @@ int autotune(ibgpu_batch *b) {
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   float best = 1e30f;
-  int best_grid = grids[0], best_threads = blocks[0];
   if (b->nstages == 1)
     fast::launch_stage_input_batch(b->d_args, b->d_work[r], b->nwork[r], b->stream);
   for (int nt : blocks)
-    for (int g : grids) {
+    for (int g : grids_of(nt)) {
       float tbest = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
         CK(cudaEventRecord(e0, b->stream));

@@ -1038,6 +1038,12 @@ void launch_stage_input(const StageArgs &a, int ntiles, cudaStream_t st, bool de
 }
 
 #ifdef IBGPU_FAST_BUILD
+int stage_resident_ctas(bool mixed, int threads) {
+  const bool ninth = threads > kTileCells;
+  if (mixed) return ninth ? stage_min_blocks<float, kTileCells + 32>() : stage_min_blocks<float, kTileCells>();
+  return ninth ? stage_min_blocks<double, kTileCells + 32>() : stage_min_blocks<double, kTileCells>();
+}
+
 // the same over a batch's work list (one-stage schemes: one StageArgs a case)
 __global__ void __launch_bounds__(kTileCells)
     stage_input_batch(const StageArgs *__restrict__ args, const int2 *__restrict__ work) {

@@ -53,6 +53,8 @@ void launch_stage_batch(const StageArgs *args, const CaseConst *ccs, const int2 
                         int stage, int nstages, const int *phase_base, int limiter, bool visc,
                         bool final_stage, bool mixed, int grid, int threads, int table,
                         cudaStream_t st);
+// CTAs per SM that the (batched) stage kernel's registers are bounded for
+int stage_resident_ctas(bool mixed, int threads);
 void launch_stage_input_batch(const StageArgs *args, const int2 *work, int nwork, cudaStream_t st);
 // constant-memory table of batched stage arguments: reserve a byte range on
 // a device (16-byte aligned offset, -1 when it does not fit), release it,

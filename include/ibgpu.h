@@ -451,8 +451,9 @@ void ibgpu_destroy(ibgpu_ctx *ctx);
  * schedule phase in a CUDA graph and replayed; the captures happen at the
  * start of the first run.  On the first run an
  * autotuner times the candidate shapes of the merged stage launch (CTA
- * count: one CTA per work item or 1-4 / 1-6 persistent CTAs per SM; block:
- * 256 or 288 threads) and keeps the fastest.  The cases must agree on precision (IBGPU_FP64 or
+ * count: one CTA per work item or 1-4 persistent CTAs per SM (1-5 in the
+ * mixed build with 256 threads); block: 256 or 288 threads) and keeps the
+ * fastest.  The cases must agree on precision (IBGPU_FP64 or
  * IBGPU_MIXED), limiter, viscosity, stage count and coefficients; their CFL
  * intervals (dt_var_step) may differ when each divides the longest marching
  * step of the batch (each case then takes its CFL pass on its own steps, as

@@ -95,3 +95,17 @@ def test_allocation_free_final_stage_reads_no_field_it_writes(api, precision, ns
     step(lambda: api.ib.step_periodic_noalloc(P, 0, 48, 48, rows.ctypes.data, rows.ctypes.data, 1.0))
     stages = api.launches("stage_kernel")
     assert len(stages) == nstages and not races(stages[-1][2])
+
+
+@pytest.mark.parametrize("precision,resident", [("FP64", {256: 4, 288: 4}), ("MIXED", {256: 5, 288: 4})])
+def test_tuning_times_resident_grids_only(api, precision, resident):
+    s = solver(api, 512, getattr(api.ib, precision), 3)  # 1024 tiles
+    b = api.ib.Batch([s])
+    b.run(0, 1)
+    tuned = {}
+    for grid, threads, _ in b.info()["tuning"]:
+        tuned.setdefault(threads, []).append(grid)
+    # one CTA per item, then persistent ones on 148 multiprocessors
+    assert tuned == {t: [148 * m for m in range(n + 1)] for t, n in resident.items()}
+    b.close()
+    s.close()
