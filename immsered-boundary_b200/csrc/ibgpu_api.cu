@@ -1862,7 +1862,7 @@ int update_fills(ibgpu_batch *b) {
   bool same = b->lists.size() == b->cases.size();
   for (size_t i = 0; same && i < b->cases.size(); ++i) same = b->lists[i] == b->cases[i]->lists;
   if (same) return IBGPU_OK;
-  if (b->stream) CK(cudaStreamSynchronize(b->stream));
+  CK(cudaStreamSynchronize(b->stream));
   b->drop_graphs();
   b->drop_fills();
   const int rc = build_fills(b);
@@ -2093,14 +2093,12 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
     if ((rc = autotune(b))) return rc;
     b->drop_graphs();  // captured with the previous launch shape
   }
-  // merged launches, captured where the stream can be (the legacy one
-  // cannot); a case with kernel timing enabled, and schedules that repeat too
-  // rarely, take each case's own launches
-  bool merged = b->full_period <= kMaxBatchPeriod;
-  for (int i = 0; i < n; ++i) merged = merged && !b->cases[i]->timing;
-  if (merged && (rc = update_fills(b))) return rc;
-  const bool use_graphs = merged && b->stream != nullptr && !b->timing;
-  if (use_graphs && (rc = batch_prepare_graphs(b))) return rc;
+  // merged launches, captured in a graph per step; with timing of the stages
+  // or of a case's kernels, and for schedules that repeat too rarely, each
+  // case's own launches
+  bool use_graphs = b->full_period <= kMaxBatchPeriod && !b->timing;
+  for (int i = 0; i < n; ++i) use_graphs = use_graphs && !b->cases[i]->timing;
+  if (use_graphs && ((rc = update_fills(b)) || (rc = batch_prepare_graphs(b)))) return rc;
   for (int i = 0; i < n; ++i) {
     if (b->cases[i]->download_pending) {
       CK(cudaStreamWaitEvent(st, b->cases[i]->ev_copied, 0));
@@ -2128,8 +2126,6 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
       cudaGraphExec_t gx = nullptr;
       if ((rc = batch_step_graph(b, ts % b->full_period, cfl, &gx))) return rc;
       CK(cudaGraphLaunch(gx, st));
-    } else if (merged && !b->timing) {
-      if ((rc = enqueue_batch_step(b, ts % b->full_period, cfl, st))) return rc;
     } else {
       fast::launch_batch_step(b->d_phase_base, b->d_args, n, b->nstages, st);
       for (int i = 0; i < n; ++i) {

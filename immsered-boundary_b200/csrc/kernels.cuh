@@ -340,10 +340,6 @@ struct SRec<float> {
   static __device__ __forceinline__ void st(V *a, int i, int, float x, float y, float z, float w) {
     a[i] = make_float4(x, y, z, w);
   }
-  // half h of record i: components 2h, 2h + 1
-  static __device__ __forceinline__ void st_half(V *a, int i, int, int h, float x, float y) {
-    reinterpret_cast<float2 *>(a + i)[h] = make_float2(x, y);
-  }
 };
 
 template <>
@@ -359,6 +355,7 @@ struct SRec<double> {
     a[i] = make_double2(x, y);
     a[i + n] = make_double2(z, w);
   }
+  // half h of record i: components 2h, 2h + 1
   static __device__ __forceinline__ void st_half(V *a, int i, int n, int h, double x, double y) {
     a[i + h * n] = make_double2(x, y);
   }
