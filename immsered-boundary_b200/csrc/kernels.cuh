@@ -37,9 +37,6 @@ __device__ __forceinline__ void step_reset(const StageArgs &a) {
   }
 }
 
-// Threads of a fast-build stage CTA: FP64 adds a ninth warp that owns the
-// tile's east/north edge faces and outer slopes, so every warp computes two
-// faces; FP32 keeps 8 warps (its face work is cheap enough).
 // Whether a thread evaluates its two faces as one paired flux: FP32 yes
 // (f32x2 instructions); FP64 no (interleaving two scalar chains needs
 // registers that cost more occupancy than the extra independence returns).
@@ -54,15 +51,23 @@ constexpr bool kPairFaces = sizeof(R) == 4;
 template <typename R>
 constexpr bool kHalfHalo = sizeof(R) == 8;
 
+// Threads of a fast-build stage CTA: FP64 adds a ninth warp that owns the
+// tile's east/north edge faces and outer slopes, so every warp computes two
+// faces; FP32 keeps 8 warps (its face work is cheap enough).
 template <typename R>
 struct StageThreads {
   static constexpr int value = sizeof(R) == 8 ? 288 : kTileCells;
 };
 
 // Resident CTAs per SM the register budget is fixed for, by arithmetic and
-// block shape (the batched stage tunes between 256 and 288 threads).  FP64
-// 56 registers; FP32 48, as 40 (six CTAs) spilled: 20 steps of the 2048^2
-// vortex 8.80 ms with six, 8.35 with five, 9.14 with four.
+// block shape (the batched stage tunes between 256 and 288 threads).  FP64:
+// 56 registers, 24-30 bytes of spill stores per thread.  FP32, 256 threads:
+// 48 registers, which spill too (van Leer 80-108 bytes, minmod 24-56); the
+// measured best all the same: 20 steps of the 2048^2 vortex 8.80 ms with six
+// CTAs (40 registers), 8.35 with five, 9.14 with four.  With 288 threads four
+// CTAs have 56 registers; the batched kernel then spills next to nothing (0-4
+// bytes with its arguments in constant memory).  That shape is not timed for
+// the single case.
 template <typename R, int NT>
 constexpr int stage_min_blocks() {
   return sizeof(R) == 8 ? 4 : (NT > kTileCells ? 4 : 5);
@@ -74,8 +79,9 @@ constexpr int stage_min_blocks() {
 // global value first to skip it put a memory round trip on the tail of
 // every CTA: 29 us per FP64 2048^2 final stage).  Components map to
 // res_max[0,1,2,4] (no z momentum in 2-D).
-// Every thread of the block must call it; sred is shared scratch of 32
-// words that no thread reads or writes any more.
+// Every thread of the block must call it; sred is shared scratch of 4 NT / 32
+// words that no thread reads or writes any more (with the fold below, which
+// uses words 64 to 64 + NT / 32, that many).
 template <int NT = kTileCells>
 __device__ __forceinline__ void block_resnorm(const unsigned long long (&rb)[4], DevDiag *d,
                                               unsigned long long *sred) {

@@ -474,7 +474,7 @@ int ibgpu_batch_run(ibgpu_batch *b, int ts0, int nsteps, double *dt, ibgpu_diag 
  * autotuner at the next run (the default). */
 int ibgpu_batch_set_grid(ibgpu_batch *b, int grid);
 /* Threads per CTA of the merged stage launches from the next run on: 256
- * (the tile's edge faces on its first two warps) or 288 (a ninth warp owns
+ * (the tile's edge faces on its first warp) or 288 (a ninth warp owns
  * them), 0 = chosen by the autotuner at the next run (the default; it times
  * both with every CTA count it tries).  The same results either way. */
 int ibgpu_batch_set_block(ibgpu_batch *b, int threads);
@@ -511,8 +511,9 @@ void ibgpu_batch_destroy(ibgpu_batch *b);
  * must be multiples of 16 with nx * ny <= IBGPU_NOALLOC_MAX_CELLS, else
  * IBGPU_E_ARG.  The first call on a device looks up that array's address
  * and registers one static host page that returns dt and diag (once per
- * device, with the device current): make it before any stream capture.  All calls share the array, which keeps the last call's contents;
- * calls that overlap on the GPU race, so the caller serialises them.  The
+ * device, with the device current; registered until the process exits): make
+ * it before any stream capture.  All calls share the array, which keeps the
+ * last call's contents; calls that overlap on the GPU race, so the caller serialises them.  The
  * call synchronises `stream` (a cudaStream_t, NULL for the legacy stream)
  * to return dt and diag. */
 #define IBGPU_NOALLOC_MAX_CELLS 65536
